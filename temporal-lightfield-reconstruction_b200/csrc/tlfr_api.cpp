@@ -1054,9 +1054,10 @@ tlfr_status tlfr_tree_export(tlfr_ctx* ctx, float* nodef, int* nodei, float* sam
         if (nodef)
         {
             float* f = nodef + (size_t)i * 14;
-            f[0] = n.a.x; f[1] = n.a.y; f[2] = n.a.z; f[3] = n.a.w;
-            f[4] = n.b.x; f[5] = n.b.y; f[6] = n.b.z; f[7] = n.b.w;
-            f[8] = n.c.x; f[9] = n.c.y; f[10] = n.c.z; f[11] = n.c.w;
+            f[0] = n.a.x; f[1] = n.a.z; f[2] = n.b.x;
+            f[3] = n.a.y; f[4] = n.a.w; f[5] = n.b.y;
+            f[6] = n.b.z; f[7] = n.c.x; f[8] = n.c.z;
+            f[9] = n.b.w; f[10] = n.c.y; f[11] = n.c.w;
             f[12] = ts[i].x; f[13] = ts[i].y;
         }
         if (nodei)

@@ -848,16 +848,16 @@ __device__ __forceinline__ float bnode_cost(const BNode& n)
     return bounds_cost(b, n.ns);
 }
 
-__device__ __forceinline__ QNode to_qnode(const BNode& n)
+__device__ __forceinline__ QNode to_qnode(const BNode& n, int slot)
 {
     QNode q;
-    q.a = make_float4(n.p[0], n.p[1], n.p[2], n.p[3]);
-    q.b = make_float4(n.p[4], n.p[5], n.p[6], n.p[7]);
-    q.c = make_float4(n.p[8], n.p[9], n.p[10], n.p[11]);
+    q.a = make_float4(n.p[0], n.p[3], n.p[1], n.p[4]);
+    q.b = make_float4(n.p[2], n.p[5], n.p[6], n.p[9]);
+    q.c = make_float4(n.p[7], n.p[10], n.p[8], n.p[11]);
     if (n.ref < 0)
     {
         int s0 = ~n.ref;
-        q.d = make_int4(-1, -1, s0, s0 + n.ns);
+        q.d = make_int4(~slot, -1, s0, s0 + n.ns);
     }
     else
         q.d = make_int4(n.ref, n.ref + 1, -1, -1);
@@ -866,7 +866,7 @@ __device__ __forceinline__ QNode to_qnode(const BNode& n)
 
 __device__ __forceinline__ void store_node(QNode* nodes, float2* tspans, int slot, const BNode& n)
 {
-    nodes[slot] = to_qnode(n);
+    nodes[slot] = to_qnode(n, slot);
     tspans[slot] = make_float2(n.tspan[0], n.tspan[1]);
 }
 

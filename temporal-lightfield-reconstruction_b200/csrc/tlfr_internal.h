@@ -17,10 +17,12 @@ namespace tlfr
 {
 
 // Hierarchy node as the query reads it: 64 bytes, one aligned 64-byte load.
-//   a = (xmin.t, xmin.uv, xmin.c, xmax.t)
-//   b = (xmax.uv, xmax.c, ymin.t, ymin.uv)
-//   c = (ymin.c, ymax.t, ymax.uv, ymax.c)
-//   d = (child0 or -1 for a leaf, child1, s0, s1)
+//   a = (xmin.t, xmax.t, xmin.uv, xmax.uv)
+//   b = (xmin.c, xmax.c, ymin.t, ymax.t)
+//   c = (ymin.uv, ymax.uv, ymin.c, ymax.c)
+//   d = (child0, or ~node for a leaf, child1, s0, s1)
+// Opposite planes' coefficients lie side by side: both are evaluated with packed
+// operations.
 // Internal nodes' children are emitted as a pair, so child1 == child0 + 1.
 struct __align__(16) QNode
 {

@@ -29,7 +29,9 @@
 #include "tlfr_common.cuh"
 #include "tlfr_internal.h"
 
+#include <algorithm>
 #include <array>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -63,6 +65,8 @@ struct QParams
     float c0, c1;               // refocused CoC coefficients
     float disp0;
     int   lens_filter, time_filter;
+    float r2_wide, min_w;       // may_accept()'s bounds at 1R (accept_bound())
+    float one;                  // 1 (eval2())
     const unsigned char* route_fast;   // per pixel, nonzero: first-surface fast path (or null)
 };
 
@@ -114,6 +118,71 @@ TLFR_HD QNode load_node(const QNode* nodes, int i)
 #endif
 }
 
+#ifdef __CUDACC__
+// Pairs of floats in one register pair, for the packed operations (each half
+// rounded as the scalar operation).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// A node's planes as (min, max) pairs, and its link.
+struct NodePairs
+{
+    f32x2 xt, xu, xc, yt, yu, yc;
+    int link, s0, s1;
+};
+__device__ __forceinline__ NodePairs load_pairs(const QNode* nodes, int i)
+{
+    NodePairs n;
+    const QNode* p = nodes + i;
+    f32x2 d0, d1;
+    asm("ld.global.v4.b64 {%0,%1,%2,%3}, [%4];" : "=l"(n.xt), "=l"(n.xu), "=l"(n.xc), "=l"(n.yt) : "l"(p));
+    asm("ld.global.v4.b64 {%0,%1,%2,%3}, [%4];"
+        : "=l"(n.yu), "=l"(n.yc), "=l"(d0), "=l"(d1) : "l"(reinterpret_cast<const char*>(p) + 32));
+    n.link = (int)(unsigned)d0;
+    n.s0 = (int)(unsigned)d1;
+    n.s1 = (int)(unsigned)(d1 >> 32);
+    return n;
+}
+// plane_eval of a (min, max) pair of planes at (t, uv).  ptxas 12.9 contracts a
+// packed multiplication and addition into one rounding, .rn and --fmad=false
+// notwithstanding (2.4% of random planes differed from plane_eval in the last
+// bit), so the products are added through a multiplication by a one that it
+// cannot see (QParams::one): same instruction count, each step rounded.
+__device__ __forceinline__ f32x2 eval2(f32x2 pt, f32x2 pu, f32x2 pc, f32x2 t, f32x2 uv, f32x2 one)
+{
+    f32x2 s;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(s) : "l"(mul2(t, pt)), "l"(one), "l"(mul2(pu, uv)));
+    return add2(s, pc);
+}
+#endif
+
 struct LeafSort
 {
     Leaf* l;
@@ -123,10 +192,10 @@ struct LeafSort
 
 TLFR_HD void node_planes(const QNode& n, float (&p)[4][3])
 {
-    p[0][0] = n.a.x; p[0][1] = n.a.y; p[0][2] = n.a.z;
-    p[1][0] = n.a.w; p[1][1] = n.b.x; p[1][2] = n.b.y;
-    p[2][0] = n.b.z; p[2][1] = n.b.w; p[2][2] = n.c.x;
-    p[3][0] = n.c.y; p[3][1] = n.c.z; p[3][2] = n.c.w;
+    p[0][0] = n.a.x; p[0][1] = n.a.z; p[0][2] = n.b.x;
+    p[1][0] = n.a.y; p[1][1] = n.a.w; p[1][2] = n.b.y;
+    p[2][0] = n.b.z; p[2][1] = n.c.x; p[2][2] = n.c.z;
+    p[3][0] = n.b.w; p[3][1] = n.c.y; p[3][2] = n.c.w;
 }
 
 // sameSurface (Reconstruction.hpp:457-525)
@@ -162,10 +231,10 @@ TLFR_HD bool same_surface(const QNode& n0, const QNode& n1, const float* uvtmin,
 // Node::intersect (Reconstruction.hpp:204-216)
 TLFR_HD bool node_intersect(const QNode& n, const Query& o, float R)
 {
-    float mnx = ((o.t * n.a.x + n.a.y * o.u) + n.a.z) - R;
-    float mny = ((o.t * n.b.z + n.b.w * o.v) + n.c.x) - R;
-    float mxx = ((o.t * n.a.w + n.b.x * o.u) + n.b.y) + R;
-    float mxy = ((o.t * n.c.y + n.c.z * o.v) + n.c.w) + R;
+    float mnx = ((o.t * n.a.x + n.a.z * o.u) + n.b.x) - R;
+    float mny = ((o.t * n.b.z + n.c.x * o.v) + n.c.z) - R;
+    float mxx = ((o.t * n.a.y + n.a.w * o.u) + n.b.y) + R;
+    float mxy = ((o.t * n.b.w + n.c.y * o.v) + n.c.w) + R;
     return (o.x >= mnx && o.y >= mny && o.x <= mxx && o.y <= mxy);
 }
 
@@ -612,146 +681,227 @@ __device__ void flush_stats(const QStats& st, DevStats* ds)
 constexpr int kBlock = 128;
 // capacities of the full per-query path (statistics pass and heavy pass)
 constexpr int kStackCap = 96, kLeafCap = 256, kRsCap = 512, kSurfCap = 64;
-// capacities of the light pass: traversal stack and leaf list per output
-// sample, both in shared memory.  kLLeaf is also the most leaves the warp's
-// scan holds (one per lane).  The single-frame path runs a first light pass
-// with fewer leaves (kL1Leaf), which fits seven blocks per SM, and retries the
-// output samples that outgrow it with the full kLLeaf and a deeper stack.
-constexpr int kLStack = 16, kLLeaf = 32;
-constexpr int kL1Stack = 12, kL1Leaf = 24;
-constexpr int kL2Stack = 30, kL2Leaf = 32;
+// Capacities of the light pass: leaves and traversal stack entries per output
+// sample.  Leaves are lanes in the warp's scan, so 32 is the most it holds.  A
+// first tier with fewer leaves fits more blocks per SM; the output samples that
+// outgrow it are retried with 32 leaves and a deeper stack.  The router's
+// coarse pass counts what outgrows 32 leaves and 16 stack entries as needing
+// the full path, so its capacities are part of its features' values.
+constexpr int kProbeStack = 16, kProbeLeaf = 32;
+constexpr int kL1Stack = 24, kL1Leaf = 24;
+constexpr int kL2Stack = 32, kL2Leaf = 32;
 
-// Per-thread column of a shared-memory array laid out [slot][thread]: a warp
-// whose lanes touch different slots still hits distinct banks.  The host build
-// (stride 1) runs the same code on a plain array.
-template <class T>
-struct Column
+// Samples the scan sets aside for exact tests, per warp, from at most
+// kLightSlots output samples.
+constexpr int kLightEntries = 192;
+constexpr int kLightSlots = 8;
+
+// Working storage of one warp of the light pass.  The traversal and the sort use
+// one column per lane ([row][lane]: no bank conflicts wherever the lanes are in
+// their columns); then each row of leaves is permuted to [row][lane ^ row], so
+// that the warp reads one lane's column without conflicts.
+constexpr unsigned kUnsure = 0xffffffffu;
+template <int LEAF>
+struct LightScan
 {
-    T* base;
-    int stride;
-    TLFR_HD T& operator[](int k) const { return base[k * stride]; }
+    float          values[2][16];               // sameSurface values of the leaf under test
+    // samples set aside: the tree-ordered sample, and its leaf, slot << 5 and its output sample's
+    // lane << 8, then its tent weight, minus the distance where that is not positive, or 0
+    int2           entry[kLightEntries];
+    unsigned       conflict[kLightSlots][LEAF]; // earlier leaves that leaf k is not one surface with, or kUnsure
+    int            first_leaf[kLightSlots];     // leaf of the first accepted sample, 32 before there is one
+    int            seen[kLightSlots];           // quadrants, 16 once a second surface has opened, 32 if that is unsure
 };
-
-TLFR_HD float int_as_float_bits(int v)
-{
-#ifdef __CUDA_ARCH__
-    return __int_as_float(v);
-#else
-    float f;
-    memcpy(&f, &v, 4);
-    return f;
-#endif
-}
-TLFR_HD int float_as_int_bits(float v)
-{
-#ifdef __CUDA_ARCH__
-    return __float_as_int(v);
-#else
-    int i;
-    memcpy(&i, &v, 4);
-    return i;
-#endif
-}
-
-// A leaf found by the light pass's traversal: (sort key = w at the output
-// sample's time (RO.cpp:390-392), node index as bits).
-struct LLeafSort
-{
-    Column<float2> l;
-    TLFR_HD int cmp(int a, int b) const { const float ka = l[a].x, kb = l[b].x; return (ka < kb) ? -1 : (ka > kb) ? 1 : 0; }
-    TLFR_HD void swap(int a, int b) { const float2 t = l[a]; l[a] = l[b]; l[b] = t; }
-};
-TLFR_HD int leaf_node(const Column<float2>& leaves, int k) { return float_as_int_bits(leaves[k].y); }
-
-// Appends leaf node ni (first sample s0) with its key; false when full.
-TLFR_HD bool leaf_append(const QParams& P, const Query& o, const Column<float2>& leaves, int cap, int& nleaves, int ni,
-                         int s0)
-{
-    if (nleaves == cap)
-        return false;
-    const float4 sp0 = P.s_rec[2 * (s0)];
-    const float mvw = P.s_rec[2 * (s0) + 1].z;
-    leaves[nleaves++] = make_float2(sp0.z + (o.t - sp0.w) * mvw, int_as_float_bits(ni));
-    return true;
-}
-
-// collectInputSamples2's traversal and leaf sort (RO.cpp:368-407) for one output
-// sample at radius R: DFS in the reference's order (push child0, child1, pop the
-// last) into the leaf column, then FW::sort of the leaves by key.  Children are
-// stored as pairs, so a node that intersects has both children loaded and
-// tested together and only those that intersect are pushed (a leaf child waits
-// on the stack only behind an internal child1).  The loop has no early exit (an
-// overflow sets a flag), so a warp reconverges at the end of every step.
-// Returns the leaf count, or -1 when the stack or the leaf column is full.
-TLFR_HD int collect_pairs(const QParams& P, const Column<int>& stack, int stack_cap, const Column<float2>& leaves,
-                          int leaf_cap, const Query& o, float R)
-{
-    int nleaves = 0, sp = 0;
-    bool ok = true;
-    {
-        const QNode rn = load_node(P.nodes, P.root);
-        if (node_intersect(rn, o, R))
-        {
-            if (rn.d.x < 0)
-                ok = leaf_append(P, o, leaves, leaf_cap, nleaves, P.root, rn.d.z);
-            else
-                stack[sp++] = rn.d.x;
-        }
-    }
-    // stack entries: >= 0 the first child of an intersecting internal node;
-    // < 0 (~node) an intersecting leaf
-    while (sp > 0 && ok)
-    {
-        const int e = stack[--sp];
-        if (e < 0)
-            ok = leaf_append(P, o, leaves, leaf_cap, nleaves, ~e, P.nodes[~e].d.z);
-        else
-        {
-            const QNode n0 = load_node(P.nodes, e);
-            const QNode n1 = load_node(P.nodes, e + 1);
-            const bool h0 = node_intersect(n0, o, R);
-            const bool h1 = node_intersect(n1, o, R);
-            if (h1 && n1.d.x >= 0)
-            {
-                // child1's subtree comes first; child0 waits below it
-                if (sp + 2 > stack_cap)
-                    ok = false;
-                else
-                {
-                    if (h0)
-                        stack[sp++] = n0.d.x >= 0 ? n0.d.x : ~e;
-                    stack[sp++] = n1.d.x;
-                }
-            }
-            else
-            {
-                if (h1)
-                    ok = leaf_append(P, o, leaves, leaf_cap, nleaves, e + 1, n1.d.z);
-                if (h0 && ok)
-                {
-                    if (n0.d.x < 0)
-                        ok = leaf_append(P, o, leaves, leaf_cap, nleaves, e, n0.d.z);
-                    else if (sp + 1 > stack_cap)
-                        ok = false;
-                    else
-                        stack[sp++] = n0.d.x;
-                }
-            }
-        }
-    }
-    if (!ok)
-        return -1;
-    LLeafSort ls{ leaves };
-    fw_sort(ls, 0, nleaves);
-    return nleaves;
-}
-
-// Light pass, part 1: each lane collects its own output sample's leaves at 1R.
 template <int LEAF, int STACK>
-TLFR_HD int light_collect(const QParams& P, const Column<int>& stack, const Column<float2>& leaves, const Query& o)
+struct LightShared
+{
+    alignas(16) float query[32][5];     // the lanes' output samples
+    alignas(16) int leaf[LEAF][32];
+    union
+    {
+        int   stack[STACK][32];
+        float key[LEAF][32];
+        LightScan<LEAF> scan;
+    };
+};
+
+// One lane's leaves as FW::sort sees them: keys (w at the output sample's time,
+// RO.cpp:390-392) and nodes.
+struct LaneLeaves
+{
+    int   (*node)[32];
+    float (*key)[32];
+    int lane;
+    __device__ float& k(int i) const { return key[i][lane]; }
+    __device__ int& n(int i) const { return node[i][lane]; }
+    __device__ int cmp(int a, int b) const { const float ka = k(a), kb = k(b); return (ka < kb) ? -1 : (ka > kb) ? 1 : 0; }
+    __device__ void swap(int a, int b)
+    {
+        const float t = k(a); k(a) = k(b); k(b) = t;
+        const int m = n(a); n(a) = n(b); n(b) = m;
+    }
+};
+
+// fw_insertion_sort with the moving element held in registers: the same
+// permutation as its adjacent swaps.
+__device__ __forceinline__ void fw_insertion_sort(LaneLeaves& a, int start, int size)
+{
+    for (int i = start + 1; i < start + size; i++)
+    {
+        const float v = a.k(i);
+        const int nv = a.n(i);
+        int j = i - 1;
+        for (; j >= start; j--)
+        {
+            const float kj = a.k(j);
+            if (!(kj > v))
+                break;
+            a.k(j + 1) = kj;
+            a.n(j + 1) = a.n(j);
+        }
+        a.k(j + 1) = v;
+        a.n(j + 1) = nv;
+    }
+}
+
+// collectInputSamples2's traversal and leaf sort (RO.cpp:368-407), each lane for
+// its own output sample o at radius R (lanes without one pass valid = false): DFS
+// in the reference's order (push child0, child1, pop the last), then FW::sort of
+// the leaves by key.  Returns the leaf count, -1 when a capacity was exceeded,
+// -2 for lanes without an output sample.
+// Children are stored as pairs of 128 bytes, so a node that intersects has both
+// tested together, and only those that intersect go on: child1 next, in a
+// register, while child0 waits on the stack (links: the first child of an
+// internal node, ~node for a leaf).  The lanes' paths part after a few levels,
+// and each load then costs an L1 wavefront per four lanes at best and per line at
+// worst, so two lanes share an output sample, one per child, in two rounds: half
+// the wavefronts of a lane per output sample for a quarter more instructions
+// (960x540x8, both tiers: 166.1 ms against 172.9 with a lane per output sample).
+// Above that, down to the first node where the lanes part, there is one lane per
+// output sample and no stack.
+// All lanes take each step together; the keys are read after the traversal, as
+// neighbouring lanes reach their leaves at different steps.
+template <bool PROBE, int LEAF, int STACK>
+__device__ __forceinline__ int light_collect(const QParams& P, const Query& o, float R, bool valid,
+                                             LightShared<LEAF, STACK>& S)
 {
     static_assert(LEAF <= 32, "the warp's scan holds one leaf per lane");
-    return collect_pairs(P, stack, STACK, leaves, LEAF, o, P.disp0);
+    constexpr int kNone = (int)0x80000000;
+    const int lane = threadIdx.x & 31, child = lane & 1;
+    const f32x2 one = pack2(P.one, P.one);
+    auto hit = [R, one](const NodePairs& n, const Query& q) {
+        const f32x2 t = pack2(q.t, q.t), r = pack2(-R, R);
+        float x0, x1, y0, y1;
+        unpack2(add2(eval2(n.xt, n.xu, n.xc, t, pack2(q.u, q.u), one), r), x0, x1);
+        unpack2(add2(eval2(n.yt, n.yu, n.yc, t, pack2(q.v, q.v), one), r), y0, y1);
+        return q.x >= x0 && q.y >= y0 && q.x <= x1 && q.y <= y1;
+    };
+    int start = kNone;
+    if (valid)
+    {
+        const NodePairs rn = load_pairs(P.nodes, P.root);
+        if (hit(rn, o))
+            start = rn.link;
+    }
+    // the top of the tree, where all lanes go the same way: one lane per output
+    // sample, no stack
+    const unsigned lanes = __ballot_sync(0xffffffffu, valid);
+    if (lanes && __all_sync(0xffffffffu, start >= 0 || !valid))
+    {
+        int node = __shfl_sync(0xffffffffu, start, __ffs(lanes) - 1);
+        while (node >= 0)
+        {
+            const NodePairs n0 = load_pairs(P.nodes, node);
+            const NodePairs n1 = load_pairs(P.nodes, node + 1);
+            const unsigned m0 = __ballot_sync(0xffffffffu, valid && hit(n0, o));
+            const unsigned m1 = __ballot_sync(0xffffffffu, valid && hit(n1, o));
+            if (!((m0 == lanes && !m1) || (m1 == lanes && !m0)))
+                break;
+            node = m0 ? n0.link : n1.link;
+            start = node;
+        }
+        if (!valid)
+            start = kNone;
+    }
+    int result = 0;
+    for (int half = 0; half < 2; half++)
+    {
+        const int col = half * 16 + (lane >> 1);    // the pair's output sample: its lane and column
+        const float* qp = S.query[col];
+        const Query oc{ qp[0], qp[1], qp[2], qp[3], qp[4] };
+        int cur = __shfl_sync(0xffffffffu, start, col);
+        int count = 0, sp = 0;
+        bool ok = true;
+        // down to the next internal node: leaves go to the list
+        auto settle = [&]() {
+            while (cur < 0)
+            {
+                if (cur != kNone)
+                {
+                    if (count == LEAF)
+                        ok = false;
+                    else
+                        S.leaf[count++][col] = ~cur;
+                }
+                cur = kNone;
+                if (sp == 0)
+                    break;
+                cur = S.stack[--sp][col];
+            }
+        };
+        settle();
+        while (__any_sync(0xffffffffu, cur >= 0))
+        {
+            int mine = kNone;
+            if (cur >= 0)
+            {
+                const NodePairs n = load_pairs(P.nodes, cur + child);
+                if (hit(n, oc))
+                    mine = n.link;
+            }
+            const int other = __shfl_xor_sync(0xffffffffu, mine, 1);
+            if (cur >= 0)
+            {
+                const int v0 = child ? other : mine, v1 = child ? mine : other;
+                const bool both = v0 != kNone && v1 != kNone;
+                // the coarse pass's capacity: two entries for an open child1, one for child0
+                if (PROBE ? sp + (v1 >= 0 ? 2 : v0 >= 0 ? 1 : 0) > STACK : both && sp == STACK)
+                    ok = false;
+                cur = v1 != kNone ? v1 : v0;
+                if (both && ok)
+                    S.stack[sp++][col] = v0;
+                settle();
+                if (!ok)
+                    cur = kNone;
+            }
+        }
+        const int n = __shfl_sync(0xffffffffu, ok ? count : -1, 2 * (lane & 15));
+        if ((lane >> 4) == half)
+            result = n;
+    }
+    __syncwarp();
+    const int nleaves = valid && result > 0 ? result : 0;
+    LaneLeaves L{ S.leaf, S.key, lane };
+    for (int k = 0; k < nleaves; k++)
+    {
+        const int s0 = reinterpret_cast<const int4*>(P.nodes + L.n(k))[3].z;
+        float4 pos, mot;
+        load_sample(P.s_rec, s0, pos, mot);
+        L.k(k) = pos.z + (o.t - pos.w) * mot.z;
+    }
+    if (nleaves < 16)
+        fw_insertion_sort(L, 0, nleaves);
+    else
+        fw_sort(L, 0, nleaves);
+    __syncwarp();
+    const int most = __reduce_max_sync(0xffffffffu, nleaves);
+    for (int k = 0; k < most; k++)
+    {
+        const int node = S.leaf[k][lane];
+        __syncwarp();
+        S.leaf[k][lane ^ k] = node;
+    }
+    return valid ? result : -2;
 }
 
 // sameSurface's sixteen plane values of one node for one output sample: each
@@ -777,227 +927,107 @@ TLFR_HD void surf_vals(const QNode& n, const float* uvtmin, const float* uvtmax,
     s.v[7][0] = plane_eval(a[3], ta, 0.0f);        s.v[7][1] = plane_eval(a[3], tb, 0.0f);
 }
 
+// The same values as (min plane, max plane) pairs: x at (tmid, umin), (tmid,
+// umax), y at (tmid, vmin), (tmid, vmax), x at ta, tb, y at ta, tb; and the test of
+// same_surface_vals() on them (a: the leaf under test, b: an earlier one).
+struct SurfPairs { f32x2 v[8]; };
+
+__device__ __forceinline__ void surf_pairs(const NodePairs& n, const Query& o, float range, float p1, SurfPairs& s)
+{
+    const float ta = o.t - 0.5f * range, tb = o.t + 0.5f * range, tm = 0.5f * (ta + tb);
+    const float u0 = o.u - range, u1 = o.u + range, v0 = o.v - range, v1 = o.v + range;
+    const f32x2 tm2 = pack2(tm, tm), ta2 = pack2(ta, ta), tb2 = pack2(tb, tb), z2 = pack2(0.0f, 0.0f), one = pack2(p1, p1);
+    s.v[0] = eval2(n.xt, n.xu, n.xc, tm2, pack2(u0, u0), one);
+    s.v[1] = eval2(n.xt, n.xu, n.xc, tm2, pack2(u1, u1), one);
+    s.v[2] = eval2(n.yt, n.yu, n.yc, tm2, pack2(v0, v0), one);
+    s.v[3] = eval2(n.yt, n.yu, n.yc, tm2, pack2(v1, v1), one);
+    s.v[4] = eval2(n.xt, n.xu, n.xc, ta2, z2, one);
+    s.v[5] = eval2(n.xt, n.xu, n.xc, tb2, z2, one);
+    s.v[6] = eval2(n.yt, n.yu, n.yc, ta2, z2, one);
+    s.v[7] = eval2(n.yt, n.yu, n.yc, tb2, z2, one);
+}
+
+__device__ __forceinline__ bool same_surface_pairs(const SurfPairs& a, const SurfPairs& b)
+{
+    const float TH = 1 * 0.1f;
+    bool differ = false;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2)
+    {
+        float lo0, lo1, hi0, hi1;
+        unpack2(sub2(a.v[k], b.v[k]), lo0, lo1);
+        unpack2(sub2(a.v[k + 1], b.v[k + 1]), hi0, hi1);
+        differ = differ | ((lo0 <= -TH) & !(hi0 < TH)) | ((hi0 <= -TH) & !(lo0 < TH));
+        differ = differ | ((lo1 <= -TH) & !(hi1 < TH)) | ((hi1 <= -TH) & !(lo1 < TH));
+    }
+    return !differ;
+}
+
 // same_surface() from precomputed values: the two nodes differ where, for some
-// plane, one is more than the threshold below the other at one end and more
-// than the threshold above it at the other (ternaryEqual of two opposite
-// ternaryCompare results, Reconstruction.hpp:428-449, 457-525).  The test is
-// symmetric in its arguments.
+// plane, one is at least the threshold below the other at one end and at least
+// the threshold above it (or not comparable) at the other: ternaryEqual of two
+// opposite ternaryCompare results (Reconstruction.hpp:428-449, 457-525).  The
+// test is symmetric in its arguments.
 TLFR_HD bool same_surface_vals(const SurfVals& a, const SurfVals& b)
 {
     const float TH = 1 * 0.1f;
-    bool same = true;
+    bool differ = false;
 #pragma unroll
     for (int k = 0; k < 8; k++)
-        same = same && ternary_equal2(ternary_compare(a.v[k][0], b.v[k][0], TH), ternary_compare(a.v[k][1], b.v[k][1], TH));
-    return same;
+    {
+        const float d0 = a.v[k][0] - b.v[k][0];
+        const float d1 = a.v[k][1] - b.v[k][1];
+        differ = differ | ((d0 <= -TH) & !(d1 < TH)) | ((d1 <= -TH) & !(d0 < TH));
+    }
+    return !differ;
 }
 
-// Light pass, part 2 (RO.cpp:94-99, 165-304 for the common case): the 1R scan
-// of one output sample's sorted leaves by the whole warp, lanes over
-// consecutive samples of a leaf (coalesced 32-byte records).  It settles the
-// output sample when the 1R fetch ends with exactly one surface, or when the
-// first surface holds samples in all four quadrants by the time a second one
-// opens (fetch2R is false in both cases and the first surface is resolved).
-// Accepted samples update the surface state in sample order: quadrant mask,
-// first strict minimum distance, and the tent filter, summed in acceptance
-// order (the reference's filter order, RO.cpp:274-294).  At the first accepted
-// sample of a later leaf, sameSurface (Reconstruction.hpp:457-525) is tested
-// against every leaf since the surface opened (RO.cpp:465-470), lanes over
-// those leaves; when one fails the scan stops there.  All lanes call it with
-// the same arguments and get the same result: 0 with the colour in out, 1
-// when the output sample needs the 2R fetch.
-// first_surface (the learned router's fast path for pixels it marks as holding
-// a single apparent surface; no reference counterpart): when a second surface
-// opens, the first one is taken even if its samples do not cover all four
-// quadrants, where the reference would refetch at 2R.  Output samples with
-// nothing within 1R still take the full path.
-__device__ int light_scan_warp(const QParams& P, const Column<float2>& leaves, int nleaves, const Query& o,
-                               float4& out, bool first_surface = false)
+// Reprojection of sample i to the query's (u,v,t) and its squared distance
+// (RO.cpp:436-454); the same operations as collect().
+__device__ __forceinline__ float reproject(const QParams& P, int i, const Query& o, float& x, float& y)
 {
-    const int lane = threadIdx.x & 31;
-    const float R = P.disp0;
-    const float R2 = R * R;
-    const float RANGE = 1.0f / sqrtf(128.0f);
-    const float uvtmin[3] = { o.u - RANGE, o.v - RANGE, o.t - 0.5f * RANGE };
-    const float uvtmax[3] = { o.u + RANGE, o.v + RANGE, o.t + 0.5f * RANGE };
-    // sample range of leaf k, held by lane k (the leaf column holds at most 32),
-    // and F_k, its offset in the output sample's flat sequence of samples (the
-    // leaves' samples one after another in leaf order).  Lane k also holds leaf
-    // k's sameSurface values for this output sample.
-    int my_s0 = 0, my_n = 0;
-    SurfVals my_sv;
-    if (lane < nleaves)
+    float4 sp4, sm;
+    load_sample(P.s_rec, i, sp4, sm);
+    if (sm.x != 0.0f || sm.y != 0.0f || sm.z != 0.0f)
     {
-        const QNode nd = load_node(P.nodes, leaf_node(leaves, lane));
-        my_s0 = nd.d.z;
-        my_n = nd.d.w - nd.d.z;
-        surf_vals(nd, uvtmin, uvtmax, my_sv);
+        const float dt = o.t - sp4.w;
+        const float Px = sp4.x * sp4.z + sm.x * dt;
+        const float Py = sp4.y * sp4.z + sm.y * dt;
+        const float Pw = (1.0f * sp4.z) + sm.z * dt;
+        const float cr = rcp(Pw);
+        const float coc = P.c0 / Pw + P.c1;
+        x = Px * cr + o.u * coc;
+        y = Py * cr + o.v * coc;
     }
-    int my_f = my_n;
-    for (int off = 1; off < 32; off <<= 1)
+    else
     {
-        const int v = __shfl_up_sync(0xffffffffu, my_f, off);
-        if (lane >= off)
-            my_f += v;
+        x = sp4.x + o.u * sm.w;
+        y = sp4.y + o.v * sm.w;
     }
-    const int total = __shfl_sync(0xffffffffu, my_f, 31);
-    my_f -= my_n;
-    // Leaf and sample of flat index base + lane: the last leaf k with F_k <= f.
-    // Every leaf holds at least one sample (one leaf node per surface run of the
-    // build), so leaf starts are distinct: the leaves starting inside
-    // (base, base + lane] are counted from a mask of the chunk's leaf starts.
-    // All lanes call it; lanes with f >= total get an unused answer.
-    auto locate = [&](int base, int& k, int& i) {
-        const bool starts_in = lane < nleaves && my_f > base && my_f < base + 32;
-        const unsigned starts = __reduce_or_sync(0xffffffffu, starts_in ? 1u << (my_f - base) : 0u);
-        const int kfirst = __popc(__ballot_sync(0xffffffffu, lane < nleaves && my_f <= base)) - 1;
-        k = kfirst + __popc(starts & ((2u << lane) - 1u));
-        i = __shfl_sync(0xffffffffu, my_s0, k & 31) + (base + lane - __shfl_sync(0xffffffffu, my_f, k & 31));
-    };
-    // chunks of 32 consecutive flat samples, which may span several leaves; the
-    // next chunk's records are loaded while the current one is processed
-    int ck, ci;
-    locate(0, ck, ci);
-    bool cvalid = lane < total;
-    float4 cpos = make_float4(0, 0, 0, 0), cmot = cpos, ccol = cpos;
-    if (cvalid)
-    {
-        load_sample(P.s_rec, ci, cpos, cmot);
-        ccol = P.s_col[ci];
-    }
-    int nsurf = 0, lidx0 = 0, quad = 0, nearest = -1, result = -1, first_leaf = -1;
-    float minDist = kF32Max;
-    float4 acc = make_float4(0, 0, 0, 0);
-    for (int base = 0; base < total && result < 0; base += 32)
-    {
-        int nk, ni;
-        locate(base + 32, nk, ni);
-        const bool nvalid = base + 32 + lane < total;
-        float4 npos = make_float4(0, 0, 0, 0), nmot = npos, ncol = npos;
-        if (nvalid)
-        {
-            load_sample(P.s_rec, ni, npos, nmot);
-            ncol = P.s_col[ni];
-        }
-        // the current chunk
-        float dx = 0, dy = 0, dist2 = 0;
-        bool ok = false;
-        if (cvalid)
-        {
-            float x, y;
-            if (cmot.x != 0.0f || cmot.y != 0.0f || cmot.z != 0.0f)
-            {
-                const float dt = o.t - cpos.w;
-                const float Px = cpos.x * cpos.z + cmot.x * dt;
-                const float Py = cpos.y * cpos.z + cmot.y * dt;
-                const float Pw = (1.0f * cpos.z) + cmot.z * dt;
-                const float cr = rcp(Pw);
-                const float coc = P.c0 / Pw + P.c1;
-                x = Px * cr + o.u * coc;
-                y = Py * cr + o.v * coc;
-            }
-            else
-            {
-                x = cpos.x + o.u * cmot.w;
-                y = cpos.y + o.v * cmot.w;
-            }
-            dx = x - o.x;
-            dy = y - o.y;
-            dist2 = dx * dx + dy * dy;
-            ok = dist2 <= R2;
-        }
-        unsigned accm = __ballot_sync(0xffffffffu, ok);
-        if (accm)
-        {
-            const float dist = ok ? sqrtf(dist2) : __int_as_float(0x7f800000);
-            const float weight = 1 - dist / R;
-            const bool inc = ok && weight > 0;
-            const float4 pr = inc ? make_float4(ccol.x * weight, ccol.y * weight, ccol.z * weight, ccol.w * weight)
-                                  : make_float4(0, 0, 0, 0);
-            const int qbit = ok ? 1 << (((dx >= 0 ? 1 : 4) | (dy >= 0 ? 2 : 8)) & 3) : 0;
-            const unsigned incm = __ballot_sync(0xffffffffu, inc);
-            // the chunk's leaves in order, those with accepted samples
-            while (accm)
-            {
-                const int kseg = __shfl_sync(0xffffffffu, ck, __ffs(accm) - 1);
-                const bool inseg = ck == kseg;
-                const unsigned segm = __ballot_sync(0xffffffffu, inseg);
-                accm &= ~segm;
-                if (first_leaf != kseg)
-                {
-                    // first accepted sample of this leaf
-                    first_leaf = kseg;
-                    if (nsurf == 0)
-                    {
-                        nsurf = 1;
-                        lidx0 = kseg;
-                    }
-                    else
-                    {
-                        // lanes j in [lidx0, kseg) test leaf j against this leaf
-                        // (leaf indices are lanes: the column holds at most 32)
-                        SurfVals cur;
-#pragma unroll
-                        for (int a = 0; a < 8; a++)
-                        {
-                            cur.v[a][0] = __shfl_sync(0xffffffffu, my_sv.v[a][0], kseg);
-                            cur.v[a][1] = __shfl_sync(0xffffffffu, my_sv.v[a][1], kseg);
-                        }
-                        const bool sj = (lane >= lidx0 && lane < kseg) ? same_surface_vals(cur, my_sv) : true;
-                        if (!__all_sync(0xffffffffu, sj))   // a second surface opens: the first one is final
-                        {
-                            result = (quad == 0xF || first_surface) ? 0 : 1;
-                            break;
-                        }
-                    }
-                }
-                const bool sok = ok && inseg;
-                quad |= __reduce_or_sync(0xffffffffu, sok ? qbit : 0);
-                // first strict minimum in sample order (RO.cpp:494-499); distances
-                // are non-negative, so their bit patterns order as unsigned integers
-                const unsigned dbits = sok ? __float_as_uint(dist) : 0x7f800000u;
-                const unsigned mbits = __reduce_min_sync(0xffffffffu, dbits);
-                const float cmin = __uint_as_float(mbits);
-                if (cmin < minDist)
-                {
-                    const unsigned at = __ballot_sync(0xffffffffu, sok && dbits == mbits);
-                    minDist = cmin;
-                    nearest = __shfl_sync(0xffffffffu, ci, __ffs(at) - 1);
-                }
-                // tent filter products summed in sample order
-                for (unsigned mi = incm & segm; mi; mi &= mi - 1)
-                {
-                    const int src = __ffs(mi) - 1;
-                    acc.x += __shfl_sync(0xffffffffu, pr.x, src);
-                    acc.y += __shfl_sync(0xffffffffu, pr.y, src);
-                    acc.z += __shfl_sync(0xffffffffu, pr.z, src);
-                    acc.w += __shfl_sync(0xffffffffu, pr.w, src);
-                }
-            }
-        }
-        ck = nk; ci = ni; cvalid = nvalid;
-        cpos = npos; cmot = nmot; ccol = ncol;
-    }
-    if (result < 0)
-        result = (nsurf == 0) ? 1 : 0;
-    if (result != 0)
-        return result;
-    const float oow = rcp(acc.w);
-    acc.x *= oow; acc.y *= oow; acc.z *= oow; acc.w *= oow;
-    if (acc.w == 0)
-        acc = P.s_col[nearest];
-    if (P.lens_filter == 1)
-    {
-        float g = gaussian(o.u, 0.5f, 0) * gaussian(o.v, 0.5f, 0);
-        acc.x *= g; acc.y *= g; acc.z *= g; acc.w *= g;
-    }
-    if (P.time_filter == 1)
-    {
-        float g = gaussian(o.t, 0.25f, 0.5f);
-        acc.x *= g; acc.y *= g; acc.z *= g; acc.w *= g;
-    }
-    out = acc;
-    return 0;
+    const float dx = x - o.x, dy = y - o.y;
+    return dx * dx + dy * dy;
+}
+
+// Whether a sample may lie within the radius whose widened square is r2w
+// (accept_bound()): the reprojection with fused multiply-adds and the
+// hardware's reciprocal (relative error at most 2^-23) in place of two exact
+// divisions, about 17 instructions against 50.  Never false for a sample that
+// reproject() puts within the radius.  Samples whose w at the output time is
+// outside the range the bound is derived for always may.
+__device__ __forceinline__ bool may_accept(const QParams& P, const Query& o, const float4& sp4, const float4& sm,
+                                           float r2w)
+{
+    const float dt = o.t - sp4.w;
+    const float Pw = __fmaf_rn(sm.z, dt, sp4.z);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(Pw));
+    const float coc = __fmaf_rn(P.c0, r, P.c1);
+    const float Px = __fmaf_rn(sm.x, dt, sp4.x * sp4.z);
+    const float Py = __fmaf_rn(sm.y, dt, sp4.y * sp4.z);
+    const float dx = __fmaf_rn(o.u, coc, __fmaf_rn(Px, r, -o.x));
+    const float dy = __fmaf_rn(o.v, coc, __fmaf_rn(Py, r, -o.y));
+    const float d2 = __fmaf_rn(dx, dx, dy * dy);
+    return !(d2 > r2w) || !(Pw >= fmaxf(0.5f * sp4.z, P.min_w));
 }
 
 __device__ __forceinline__ Query query_of(const QParams& P, long long q)
@@ -1031,14 +1061,11 @@ __device__ __forceinline__ void warp_append(int* queue, int* count, bool pred, i
 constexpr int kQueueRestart = 1 << 30;
 
 constexpr int kProbe = 4;
-// resident light-pass blocks per SM: shared memory (40 KB per block) allows 5,
-// and a 5-block register budget (<= 102 per thread) measured 9% faster than 4.
-// The first tier (24 leaves, 12 stack entries: 30 KB) fits 7 at <= 72
-// registers (a few spilled): 1340 ms per 1920x1080x8 frame against 1378 at
-// 6 blocks with 28 leaves and 1492 with one tier; the retry tier (47 KB) 4.
-constexpr int kLightBlocksPerSM = 5;
+// Light-pass blocks per SM, by shared memory (24.5 KB per block of the first
+// tier, 32 KB of the others) and registers.
+constexpr int kProbeBlocksPerSM = 6;
 constexpr int kL1BlocksPerSM = 7;
-constexpr int kL2BlocksPerSM = 4;
+constexpr int kL2BlocksPerSM = 6;
 // Light-pass kinds: every output sample of a map, overflow to the full path
 // (kLightPlain); the same with overflow to a retry list (kLightFirst); the
 // output samples of a retry list (kLightRetry), overflow to the full path.
@@ -1098,99 +1125,374 @@ __device__ __forceinline__ bool light_query_id(const QParams& P, const LightMap&
     return x < P.W && y < P.H;
 }
 
-// Shared-memory columns of a light-pass block.
-template <int LEAF, int STACK>
-struct LightShared
-{
-    float2 leaves[LEAF][kBlock];
-    int stack[STACK][kBlock];
-};
-
-// One block iteration u of the light pass.  kLightRetry: the output samples
-// are retry[u * kBlock + thread] for indices below num_queries; kLightFirst:
-// those that outgrow the capacities are appended to retry.
+// One block iteration u of the light pass (RO.cpp:94-99, 165-304 for the common
+// case): each lane collects its own output sample's leaves at 1R, then the warp
+// scans the output samples in turn.  kLightRetry: the output samples are
+// retry[u * kBlock + thread] for indices below num_queries; kLightFirst: those
+// that outgrow the capacities are appended to retry.
+//
+// A sample settles when the 1R fetch ends with exactly one surface, or when the
+// first surface holds samples in all four quadrants by the time a second one
+// opens (fetch2R is false in both cases and the first surface is resolved); the
+// rest are queued for the full path.  On a routed pixel (the learned router's
+// fast path, no reference counterpart) the first surface is taken even if its
+// samples do not cover the quadrants; output samples with nothing within 1R
+// still take the full path.
+//
+// The scan is bound by instruction issue, so it does per tested sample only what
+// 93% of them need, and the rest once per batch of output samples:
+//   1. the warp runs over the output sample's leaves' samples as one flat
+//      sequence, 32 at a time across leaf boundaries (32-byte records, the next
+//      chunk on its way while the current one is tested), and sets aside those
+//      that may_accept();
+//   2. where they come from more than one leaf, sameSurface
+//      (Reconstruction.hpp:457-525) of each such leaf with every earlier one from
+//      the first, lanes over the earlier leaves, as bit masks;
+//   3. every kLightSlots output samples (or when the list is full), lanes over the
+//      samples set aside: the exact reprojection, radius test, tent weight and
+//      quadrant, up to the first accepted sample of a leaf that conflicts with a
+//      leaf since the surface opened (RO.cpp:465-470);
+//   4. lanes over (output sample, colour component): the tent filter summed in
+//      acceptance order (RO.cpp:274-294), four colours loaded at a time, and the
+//      nearest sample.
+// 1920x1080x8, both tiers: LIGHT_NOW ms; with every chunk's samples reprojected exactly
+// and handled leaf by leaf with their colours loaded and shuffled: 934 ms.
 template <bool PROBE, int LEAF, int STACK, int MODE>
 __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, long long u, long long num_queries,
                                            float4* __restrict__ qcol, int* __restrict__ heavy,
-                                           int* __restrict__ heavy_count, LightShared<LEAF, STACK>& sh,
+                                           int* __restrict__ heavy_count, LightShared<LEAF, STACK>& S,
                                            int* __restrict__ retry = nullptr, int* __restrict__ retry_count = nullptr)
 {
-    float2 (&sh_leaves)[LEAF][kBlock] = sh.leaves;
     const int lane = threadIdx.x & 31;
-    const int wbase = threadIdx.x & ~31;
-    const Column<int> stack{ &sh.stack[0][threadIdx.x], kBlock };
+    const unsigned below = (1u << lane) - 1u, upto = (2u << lane) - 1u;
+    LightScan<LEAF>& T = S.scan;
+    // this lane's output sample
+    long long q = 0;
+    bool valid;
+    if (MODE == kLightRetry)
     {
-        // each lane: traversal and leaf sort of its own output sample
-        long long q = 0;
-        bool valid;
-        if (MODE == kLightRetry)
+        const long long k = u * kBlock + threadIdx.x;
+        valid = k < num_queries;
+        q = valid ? retry[k] : 0;
+    }
+    else
+        valid = light_query_id(P, L, u, threadIdx.x, num_queries, q);
+    Query o{};
+    bool fast = false;
+    if (valid)
+    {
+        const long long pix = PROBE ? q / kProbe : q / P.M;
+        fast = !PROBE && P.route_fast && P.route_fast[pix];
+        o = PROBE ? make_query(P, (int)(pix % P.W), (int)(pix / P.W), (int)((q % kProbe) * P.M / kProbe))
+                  : query_of(P, q);
+    }
+    const int qid = valid ? (int)q : 0;
+    const unsigned fast_lanes = __ballot_sync(0xffffffffu, fast);
+    __syncwarp();       // the previous iteration's scan lists have been read
+    {
+        float* qp = S.query[lane];
+        qp[0] = o.x; qp[1] = o.y; qp[2] = o.u; qp[3] = o.v; qp[4] = o.t;
+    }
+    __syncwarp();
+    const int nl = light_collect<PROBE, LEAF, STACK>(P, o, P.disp0, valid, S);
+    __syncwarp();
+    // output samples that outgrew the capacities, and those that reach no leaf
+    if (PROBE)
+    {
+        if (nl == -1 || nl == 0)
+            atomicAdd(&heavy_count[qid / kProbe], 1);
+    }
+    else
+    {
+        if (MODE == kLightFirst)
         {
-            const long long k = u * kBlock + threadIdx.x;
-            valid = k < num_queries;
-            q = valid ? retry[k] : 0;
+            warp_append(retry, retry_count, nl == -1, qid);
+            warp_append(heavy, heavy_count, nl == 0, qid);
         }
         else
-            valid = light_query_id(P, L, u, threadIdx.x, num_queries, q);
-        Query o{};
-        int nl = -2;
-        const long long pix = valid ? (PROBE ? q / kProbe : q / P.M) : 0;
-        const bool fast = !PROBE && valid && P.route_fast && P.route_fast[pix];
-        if (valid)
+            warp_append(heavy, heavy_count, nl == -1 || nl == 0, nl == 0 ? qid : qid | kQueueRestart);
+    }
+
+    const float R = P.disp0;
+    const float R2 = R * R;
+    const float RANGE = 1.0f / sqrtf(128.0f);
+    const float* colours = reinterpret_cast<const float*>(P.s_col);
+    int cnt = 0, nslot = 0;         // samples set aside, slots in use
+    // lane -> (slot, colour component) and that slot's running surface state
+    const int my_slot = lane >> 2, comp = lane & 3;
+    int e0 = 0, e1 = 0, my_j = 0;   // the slot's samples set aside, its output sample's lane
+    int nearest = -1;
+    float acc = 0, min_dist = kF32Max;
+
+    unsigned todo = __ballot_sync(0xffffffffu, nl > 0);
+    bool open = false;              // the list filled up inside an output sample
+    int base = 0, kbase = 0, kfirst = 0;
+    while (todo || nslot)
+    {
+        if (!todo || open || nslot == kLightSlots || cnt > kLightEntries - 64)
         {
-            o = PROBE ? make_query(P, (int)(pix % P.W), (int)(pix / P.W), (int)((q % kProbe) * P.M / kProbe))
-                      : query_of(P, q);
-            nl = light_collect<LEAF, STACK>(P, stack, Column<float2>{ &sh_leaves[0][threadIdx.x], kBlock }, o);
-        }
-        const unsigned fast_lanes = __ballot_sync(0xffffffffu, fast);
-        __syncwarp();
-        // the warp: the 1R scan of each lane's output sample in turn
-        int code = 2;
-        float4 col = make_float4(0, 0, 0, 0);
-        for (int j = 0; j < 32; j++)
-        {
-            const int nlj = __shfl_sync(0xffffffffu, nl, j);
-            if (nlj < 0)
-                continue;
-            Query oj;
-            oj.x = __shfl_sync(0xffffffffu, o.x, j);
-            oj.y = __shfl_sync(0xffffffffu, o.y, j);
-            oj.u = __shfl_sync(0xffffffffu, o.u, j);
-            oj.v = __shfl_sync(0xffffffffu, o.v, j);
-            oj.t = __shfl_sync(0xffffffffu, o.t, j);
-            float4 c;
-            const Column<float2> lj{ &sh_leaves[0][wbase + j], kBlock };
-            const int r = light_scan_warp(P, lj, nlj, oj, c, (fast_lanes >> j) & 1u);
-            if (lane == j)
+            // 3. exact tests
+            __syncwarp();
+            for (int eb = 0; eb < cnt; eb += 32)
             {
-                code = r;
-                col = c;
+                const int e = eb + lane;
+                const int2 en = e < cnt ? T.entry[e] : make_int2(0, 0xffff);
+                const unsigned m = (unsigned)en.y;
+                const int slot = (m >> 5) & 7, k = m & 31;
+                const unsigned same_slot = __match_any_sync(0xffffffffu, m >> 5);
+                bool ok = false;
+                float w = 0;
+                int quadrant = 0;
+                if (e < cnt)
+                {
+                    const float* qp = S.query[m >> 8];
+                    const Query oe{ qp[0], qp[1], qp[2], qp[3], qp[4] };
+                    float x, y;
+                    const float d2 = reproject(P, en.x, oe, x, y);
+                    ok = d2 <= R2;
+                    if (ok)
+                    {
+                        const float dx = x - oe.x, dy = y - oe.y;
+                        const float dist = sqrtf(d2);
+                        const float weight = 1 - dist / R;
+                        w = weight > 0 ? weight : -dist;
+                        quadrant = ((dx >= 0 ? 1 : 4) | (dy >= 0 ? 2 : 8)) & 3;
+                    }
+                }
+                const unsigned okm = __ballot_sync(0xffffffffu, ok) & same_slot;
+                if (ok && lane == __ffs(okm) - 1 && T.first_leaf[slot] == 32)
+                    T.first_leaf[slot] = k;
+                __syncwarp();
+                bool stop = false, unsure = false;
+                if (ok)
+                {
+                    const int k1 = T.first_leaf[slot];
+                    const unsigned c = k != k1 ? T.conflict[slot][k] : 0u;
+                    stop = (T.seen[slot] & 16) || (c >> k1) != 0;
+                    unsure = MODE == kLightFirst && !(T.seen[slot] & 16) && c == kUnsure;
+                }
+                const unsigned stopm = __ballot_sync(0xffffffffu, stop) & same_slot;
+                // a second surface opens at the first of these: the first one is final
+                ok = ok && !(stopm && lane >= __ffs(stopm) - 1);
+                int seen = stopm ? 16 : 0;
+                if (MODE == kLightFirst)
+                {
+                    const unsigned um = __ballot_sync(0xffffffffu, unsure);
+                    if (stopm & (0u - stopm) & um)
+                        seen |= 32;
+                }
+#pragma unroll
+                for (int b = 0; b < 4; b++)
+                    if (__ballot_sync(0xffffffffu, ok && quadrant == b) & same_slot)
+                        seen |= 1 << b;
+                if (e < cnt)
+                {
+                    T.entry[e].y = __float_as_int(ok ? w : 0.0f);
+                    if (lane == __ffs(same_slot) - 1)
+                        T.seen[slot] |= seen;
+                }
+                __syncwarp();
             }
-        }
-        __syncwarp();
-        if (PROBE)
-        {
-            // heavy_count is the per-pixel count here
-            if (valid && code != 0)
-                atomicAdd(&heavy_count[pix], 1);
-            return;
-        }
-        bool hv = false, rt = false;
-        int entry = 0;
-        if (valid)
-        {
-            if (code == 0)
-                qcol[q] = col;
-            else if (MODE == kLightFirst && code == 2)
-                rt = true;
+            // 4. the tent filter in order
+            if (!PROBE)
+            {
+                constexpr int kAhead = 4;
+                for (int e = e0; e < e1; e += kAhead)
+                {
+                    float w[kAhead], c[kAhead];
+                    int i[kAhead];
+#pragma unroll
+                    for (int a = 0; a < kAhead; a++)
+                    {
+                        const int2 en = e + a < e1 ? T.entry[e + a] : make_int2(0, 0);
+                        w[a] = __int_as_float(en.y);
+                        i[a] = en.x;
+                    }
+#pragma unroll
+                    for (int a = 0; a < kAhead; a++)
+                        c[a] = w[a] > 0 ? colours[4 * (size_t)i[a] + comp] : 0.0f;
+#pragma unroll
+                    for (int a = 0; a < kAhead; a++)
+                        if (w[a] > 0)
+                            acc += c[a] * w[a];
+                        else if (w[a] < 0 && -w[a] < min_dist)      // read only where no sample has a weight
+                        {
+                            min_dist = -w[a];
+                            nearest = i[a];
+                        }
+                }
+            }
+            // finished output samples
+            const bool fin = my_slot < nslot && !(open && my_slot == nslot - 1);
+            const int seen = T.seen[my_slot];
+            const bool redo = MODE == kLightFirst && (seen & 32);
+            const bool settled = T.first_leaf[my_slot] < 32 && (seen < 16 || (seen & 15) == 15 || ((fast_lanes >> my_j) & 1u)) && !redo;
+            const int mq = __shfl_sync(0xffffffffu, qid, my_j);
+            if (PROBE)
+            {
+                if (fin && comp == 0 && !settled)
+                    atomicAdd(&heavy_count[mq / kProbe], 1);
+            }
             else
             {
-                hv = true;
-                entry = (int)q | (code == 2 ? kQueueRestart : 0);
+                const float aw = __shfl_sync(0xffffffffu, acc, lane | 3);
+                if (fin && settled)
+                {
+                    const float oow = rcp(aw);
+                    float c = acc * oow;
+                    if (aw * oow == 0)
+                        c = colours[4 * (size_t)nearest + comp];
+                    const float* qp = S.query[my_j];
+                    if (P.lens_filter == 1)
+                        c *= gaussian(qp[2], 0.5f, 0) * gaussian(qp[3], 0.5f, 0);
+                    if (P.time_filter == 1)
+                        c *= gaussian(qp[4], 0.25f, 0.5f);
+                    reinterpret_cast<float*>(qcol)[4 * (size_t)mq + comp] = c;
+                }
+                warp_append(heavy, heavy_count, fin && comp == 0 && !settled && !redo, mq);
+                if (MODE == kLightFirst)
+                    warp_append(retry, retry_count, fin && comp == 0 && redo, mq);
+            }
+            __syncwarp();
+            cnt = 0;
+            e0 = e1 = 0;
+            if (!open)
+                nslot = 0;
+            if (!todo)
+                break;
+        }
+        // the next output sample, or the rest of one the list filled up in
+        const int j = __ffs(todo) - 1;
+        const float* qj = S.query[j];
+        const Query oj{ qj[0], qj[1], qj[2], qj[3], qj[4] };
+        if (!open)
+        {
+            if (my_slot == nslot)
+            {
+                e0 = e1 = cnt;
+                my_j = j;
+                nearest = -1;
+                acc = 0;
+                min_dist = kF32Max;
+            }
+            if (lane == 0)
+            {
+                T.first_leaf[nslot] = 32;
+                T.seen[nslot] = 0;
+            }
+            nslot++;
+            base = 0;
+            kbase = -1;
+            kfirst = 32;
+        }
+        open = false;
+        const int slot = nslot - 1;
+        // 1. lane k: leaf k's sample range and its offset in the flat sequence
+        const int nlj = __shfl_sync(0xffffffffu, nl, j);
+        NodePairs leaf;
+        int my_n = 0;
+        if (lane < nlj)
+        {
+            leaf = load_pairs(P.nodes, S.leaf[lane][j ^ lane]);
+            my_n = leaf.s1 - leaf.s0;
+        }
+        int my_f = my_n;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            const int v = __shfl_up_sync(0xffffffffu, my_f, off);
+            if (lane >= off)
+                my_f += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, my_f, 31);
+        my_f = lane < nlj ? my_f - my_n : 0x7fffffff;
+        const int my_d = lane < nlj ? leaf.s0 - my_f : 0;
+        const int mine = total - lane;      // this lane's samples are below it
+        // Leaf k and sample i of flat index b + lane: every leaf holds at least one
+        // sample (one leaf node per surface run of the build), so leaf starts are
+        // distinct; kbase + 1 leaves start before the chunk.
+        auto locate = [&](int b, int& k, int& i) {
+            const unsigned at = (unsigned)(my_f - b);
+            const unsigned starts = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+            k = kbase + __popc(starts & upto);
+            kbase += __popc(starts);
+            i = b + lane + __shfl_sync(0xffffffffu, my_d, k);
+        };
+        const int first = cnt, tag = (slot << 5) | (j << 8);
+        for (;;)
+        {
+            const int kprev = kbase;
+            int ck, ci;
+            float4 cpos, cmot;
+            locate(base, ck, ci);
+            if (base < mine)
+                load_sample(P.s_rec, ci, cpos, cmot);
+            const bool may = base < mine && may_accept(P, oj, cpos, cmot, P.r2_wide);
+            const unsigned m = __ballot_sync(0xffffffffu, may);
+            if (cnt + __popc(m) > kLightEntries)
+            {
+                open = true;
+                kbase = kprev;
+                break;
+            }
+            if (may)
+            {
+                const int e = cnt + __popc(m & below);
+                T.entry[e] = make_int2(ci, ck | tag);
+            }
+            cnt += __popc(m);
+            base += 32;
+            if (base >= total)
+                break;
+        }
+        __syncwarp();
+        if (my_slot == slot)
+            e1 = cnt;
+        // 2. the leaves of the samples set aside
+        unsigned mask = 0;
+        for (int e = first + lane; e < cnt; e += 32)
+            mask |= 1u << (T.entry[e].y & 31);
+        mask = __reduce_or_sync(0xffffffffu, mask);
+        if (kfirst == 32 && mask)
+            kfirst = __ffs(mask) - 1;
+        mask &= ~(1u << (kfirst & 31));
+        if (mask)
+        {
+            SurfPairs values;
+            surf_pairs(leaf, oj, RANGE, P.one, values);
+            for (int b = 0; mask; b ^= 1)
+            {
+                // leaf k's values to all lanes, through shared memory
+                const int k = __ffs(mask) - 1;
+                mask &= mask - 1;
+                ulonglong2* row = reinterpret_cast<ulonglong2*>(T.values[b]);
+                if (lane == k)
+#pragma unroll
+                    for (int a = 0; a < 4; a++)
+                        row[a] = make_ulonglong2(values.v[2 * a], values.v[2 * a + 1]);
+                __syncwarp();
+                SurfPairs cur;
+#pragma unroll
+                for (int a = 0; a < 4; a++)
+                {
+                    const ulonglong2 v = row[a];
+                    cur.v[2 * a] = v.x;
+                    cur.v[2 * a + 1] = v.y;
+                }
+                const unsigned c = __ballot_sync(0xffffffffu, lane >= kfirst && lane < k && !same_surface_pairs(cur, values));
+                if (lane == 0)
+                    T.conflict[slot][k] = c;
+                // the scan almost surely ends at leaf k: the rest are looked at only if it does not
+                if (MODE == kLightFirst && c)
+                {
+                    if ((mask >> lane) & 1u)
+                        T.conflict[slot][lane] = kUnsure;
+                    mask = 0;
+                }
             }
         }
-        warp_append(heavy, heavy_count, hv, entry);
-        if (MODE == kLightFirst)
-            warp_append(retry, retry_count, rt, (int)q);
+        if (!open)
+            todo &= todo - 1;
     }
 }
 
@@ -1201,7 +1503,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS_PER_SM)
 k_query_light(QParams P, LightMap L, long long num_queries, float4* __restrict__ qcol, int* __restrict__ heavy,
               int* __restrict__ heavy_count, int* __restrict__ retry, int* __restrict__ retry_count)
 {
-    __shared__ LightShared<LEAF, STACK> sh;
+    __shared__ LightShared<LEAF, STACK> shw[kBlock / 32];
+    auto& sh = shw[threadIdx.x >> 5];
     if (MODE == kLightRetry)
     {
         const long long n = *retry_count;
@@ -1215,7 +1518,7 @@ k_query_light(QParams P, LightMap L, long long num_queries, float4* __restrict__
 }
 
 // the light-pass instances
-#define K_LIGHT_PLAIN(PROBE) k_query_light<PROBE, kLLeaf, kLStack, kLightBlocksPerSM, kLightPlain>
+#define K_LIGHT_PLAIN(PROBE) k_query_light<PROBE, kProbeLeaf, kProbeStack, kProbeBlocksPerSM, kLightPlain>
 #define K_LIGHT_FIRST k_query_light<false, kL1Leaf, kL1Stack, kL1BlocksPerSM, kLightFirst>
 #define K_LIGHT_RETRY k_query_light<false, kL2Leaf, kL2Stack, kL2BlocksPerSM, kLightRetry>
 
@@ -1260,32 +1563,6 @@ struct CoopScratch
 };
 
 __device__ __forceinline__ unsigned lanes_below(int lane) { return (1u << lane) - 1u; }
-
-// Reprojection of sample i to the query's (u,v,t) and its squared distance
-// (RO.cpp:436-454); the same operations as collect().
-__device__ __forceinline__ float reproject(const QParams& P, int i, const Query& o, float& x, float& y)
-{
-    float4 sp4, sm;
-    load_sample(P.s_rec, i, sp4, sm);
-    if (sm.x != 0.0f || sm.y != 0.0f || sm.z != 0.0f)
-    {
-        const float dt = o.t - sp4.w;
-        const float Px = sp4.x * sp4.z + sm.x * dt;
-        const float Py = sp4.y * sp4.z + sm.y * dt;
-        const float Pw = (1.0f * sp4.z) + sm.z * dt;
-        const float cr = rcp(Pw);
-        const float coc = P.c0 / Pw + P.c1;
-        x = Px * cr + o.u * coc;
-        y = Py * cr + o.v * coc;
-    }
-    else
-    {
-        x = sp4.x + o.u * sm.w;
-        y = sp4.y + o.v * sm.w;
-    }
-    const float dx = x - o.x, dy = y - o.y;
-    return dx * dx + dy * dy;
-}
 
 // DFS traversal into leaves[] with leaf keys (RO.cpp:368-395) and FW::sort of
 // the leaves (RO.cpp:407).  Returns the leaf count or -1 on overflow.
@@ -2713,6 +2990,30 @@ size_t slot_bytes_for(int stack_cap, int leaf_cap, int rs_cap, int surf_cap)
     return (b + 255) & ~(size_t)255;
 }
 
+// Bounds of may_accept() for a hierarchy and output setting (uvt: the override,
+// or null for the pattern, whose |u|, |v| are at most 1).  With e = 2^-24,
+// X the largest sample coordinate, O the largest output coordinate, |u|, |v| <= U,
+// w >= max(z / 2, min_w) and so D = U (|C0| / min_w + |C1|) the largest CoC term:
+// of a sample within the radius, both reprojections are within
+// (15 (|x z| + |m dt|) / w + 16 D + 3 R + 2 O) e of the real one between them, and
+// (|x z| + |m dt|) / w <= 4 X + O + D + R.  Widened by half again.
+void accept_bound(QParams& P, const Ctx& c, const float* uvt)
+{
+    const double e = 1.0 / 16777216.0, R = P.disp0;
+    double U = 1.01, X = 0;
+    if (uvt)
+        U = std::max({ U, std::fabs((double)uvt[0]), std::fabs((double)uvt[1]) });
+    for (int k = 0; k < 2; k++)
+        X = std::max({ X, std::fabs((double)c.grid.bbmin[k]), std::fabs((double)c.grid.bbmax[k]) });
+    const double O = std::max(c.W, c.H) + 1.0;
+    const double most_coc = 512.0;      // |C0| / w beyond which a sample is always tested exactly
+    P.min_w = (float)std::max(std::fabs((double)P.c0) / most_coc, 1e-30);
+    const double D = U * (most_coc * 1.001 + std::fabs((double)P.c1));
+    const double m = 1.5 * e * (64.0 * X + 20.0 * O + 36.0 * D + 24.0 * R);
+    const double r = R * (1.0 + 8.0 * e) + 1.5 * m;
+    P.r2_wide = (float)(r * r * (1.0 + 8.0 * e));
+}
+
 QParams make_params(const Ctx& c)
 {
     QParams P;
@@ -2730,6 +3031,8 @@ QParams make_params(const Ctx& c)
     P.lens_filter = c.params.lens_filter;
     P.time_filter = c.params.time_filter;
     P.route_fast = nullptr;
+    P.one = 1.0f;
+    accept_bound(P, c, c.params.override_uvt ? c.params.uvt : nullptr);
     return P;
 }
 
@@ -2842,7 +3145,8 @@ __global__ void __launch_bounds__(kBlock, FIRST ? kL1BlocksPerSM : kL2BlocksPerS
 k_batch_light(const FrameDesc* __restrict__ fd, const long long* __restrict__ unit_begin, int nframes,
               unsigned long long* __restrict__ next_unit)
 {
-    __shared__ LightShared<FIRST ? kL1Leaf : kL2Leaf, FIRST ? kL1Stack : kL2Stack> sh;
+    __shared__ LightShared<FIRST ? kL1Leaf : kL2Leaf, FIRST ? kL1Stack : kL2Stack> shw[kBlock / 32];
+    auto& sh = shw[threadIdx.x >> 5];
     __shared__ QParams sP;
     __shared__ LightMap sL;
     __shared__ long long sU;
@@ -3065,6 +3369,7 @@ tlfr_status batch_build(BatchPlan& bp, const std::vector<BatchEntry>& entries, c
             D.P.M = M;
             D.P.lens_filter = o.lens_filter;
             D.P.time_filter = o.time_filter;
+            accept_bound(D.P, c, ov ? o.uvt : nullptr);
         }
         npix[f] = (long long)c.W * c.H;
         nq[f] = npix[f] * D.P.M;
