@@ -9,10 +9,10 @@
 //   k_bucket_*        bucketing in input order (Reconstruction.cpp:605-626): counting
 //                     sort by cell, then each cell's list sorted by input index
 //   k_kd_level        buildInitialRecursive (ReconstructionTreeBuilder.cpp:34-96), one
-//                     launch per tree level
+//                     launch per tree level; k_kd_up, k_kd_offsets: counts and offsets
 //   k_entry_points    the 32 build tasks (Reconstruction.cpp:110-126, 132-143)
-//   k_leaf_prepare    per kd leaf: candidates in row-major cell order, FW::sort by (t,w),
-//                     computeTUXPlanes and the t=0/t=1 boxes (RTB.cpp:131-213)
+//   k_leaf_sort       per kd leaf: candidates in row-major cell order, FW::sort by (t,w)
+//   k_sample_prepare  per sample: computeTUXPlanes and the t=0/t=1 boxes (RTB.cpp:131-213)
 //   k_stale_boxes     a candidate with invalid bounds leaves its boxes unwritten and so
 //                     reads what earlier leaves of its task left in the reused arrays
 //                     (RTB.cpp:159-169, 184-212; Array::resize, Array.hpp:365-371, 668-692)
@@ -26,6 +26,7 @@
 #include "tlfr_common.cuh"
 #include "tlfr_internal.h"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -326,25 +327,36 @@ __device__ __forceinline__ int rect_count(const int* start, int gw, int x0, int 
     return s;
 }
 
-__global__ void k_kd_init(KdNode* kd, int* levels, GridInfo* g, int* counter)
+__global__ void k_kd_init(KdNode* kd, int* level_count, const GridInfo* g)
 {
+    if (threadIdx.x > 0)
+    {
+        if (threadIdx.x < kMaxKdLevels + 1)
+            level_count[threadIdx.x] = 0;
+        return;
+    }
     KdNode r;
     r.x0 = 0; r.y0 = 0; r.x1 = g->gw; r.y1 = g->gh;
     r.child0 = r.child1 = -1;
     r.num_samples = 0; r.depth = 0; r.path = 0; r.parent = -1;
-    r.leaf_count = 0; r.preorder_leaf = 0; r.preorder_sample = 0; r.sample_offset = 0; r.frontier = 0; r.pad = 0;
+    r.leaf_count = 0; r.preorder_leaf = 0; r.preorder_sample = 0; r.sample_offset = 0; r.frontier = 0; r.arrived = 0;
     kd[0] = r;
-    levels[0] = 0; levels[1] = 1;
-    *counter = 1;
-    g->kd_levels = 1;
+    level_count[0] = 1;
 }
 
-// Nodes of level L occupy [levels[2L], levels[2L+1]); their children are
-// allocated in pairs at the end of the node array, which becomes level L+1.
-__global__ void k_kd_level(KdNode* kd, const int* levels_in, int L, const int* __restrict__ cell_start,
-                           const GridInfo* g, int* counter)
+// First node of level L: the levels' nodes follow one another.
+__device__ __forceinline__ int level_begin(const int* level_count, int L)
 {
-    const int lo = levels_in[2 * L], hi = levels_in[2 * L + 1];
+    int lo = 0;
+    for (int l = 0; l < L; l++)
+        lo += level_count[l];
+    return lo;
+}
+
+// The nodes of level L; their children are allocated in pairs as level L + 1.
+__global__ void k_kd_level(KdNode* kd, int* level_count, int L, const int* __restrict__ cell_start, const GridInfo* g)
+{
+    const int lo = level_begin(level_count, L), hi = lo + level_count[L];
     const int gw = g->gw;
     for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
     {
@@ -361,7 +373,7 @@ __global__ void k_kd_level(KdNode* kd, const int* levels_in, int L, const int* _
             kd[i].leaf_count = 1;
             continue;
         }
-        int c = atomicAdd(counter, 2);
+        int c = hi + atomicAdd(&level_count[L + 1], 2);
         KdNode a = nd, b = nd;
         if (dx > dy)
         {
@@ -385,80 +397,89 @@ __global__ void k_kd_level(KdNode* kd, const int* levels_in, int L, const int* _
     }
 }
 
-__global__ void k_kd_next(int* levels, int L, const int* counter, GridInfo* g)
+// Sample and leaf counts of the internal nodes: every leaf climbs towards the
+// root, and the second child to arrive at a node sums it up and goes on.  One
+// launch in place of one per level (most of which held few nodes): the kd split
+// at 1280x720x8 takes 0.29 ms in 26 launches against 0.64 in 163.
+__global__ void k_kd_up(KdNode* kd, const int* level_count)
 {
-    levels[2 * (L + 1)] = levels[2 * L + 1];
-    levels[2 * (L + 1) + 1] = *counter;
-    if (levels[2 * L + 1] != *counter)
-        g->kd_levels = L + 2;
-}
-
-__global__ void k_kd_up(KdNode* kd, const int* levels, int L)
-{
-    const int lo = levels[2 * L], hi = levels[2 * L + 1];
-    for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
+    const int n = level_begin(level_count, kMaxKdLevels + 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
-        if (kd[i].child0 < 0)
+        if (kd[i].child0 >= 0)
             continue;
-        const KdNode& a = kd[kd[i].child0];
-        const KdNode& b = kd[kd[i].child1];
-        kd[i].num_samples = a.num_samples + b.num_samples;
-        kd[i].leaf_count = a.leaf_count + b.leaf_count;
+        for (int p = kd[i].parent; p >= 0; p = kd[p].parent)
+        {
+            __threadfence();
+            if (atomicAdd(&kd[p].arrived, 1) == 0)
+                break;
+            __threadfence();
+            const int a = kd[p].child0, b = kd[p].child1;
+            kd[p].num_samples = __ldcg(&kd[a].num_samples) + __ldcg(&kd[b].num_samples);
+            kd[p].leaf_count = __ldcg(&kd[a].leaf_count) + __ldcg(&kd[b].leaf_count);
+        }
     }
 }
 
-__global__ void k_kd_down(KdNode* kd, const int* levels, int L)
+// Preorder leaf and sample offsets: a node comes after the first children of the
+// ancestors on whose second side it lies.
+__global__ void k_kd_offsets(KdNode* kd, const int* level_count)
 {
-    const int lo = levels[2 * L], hi = levels[2 * L + 1];
-    for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
+    const int n = level_begin(level_count, kMaxKdLevels + 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
-        if (kd[i].child0 < 0)
-            continue;
-        KdNode& a = kd[kd[i].child0];
-        KdNode& b = kd[kd[i].child1];
-        a.preorder_leaf = kd[i].preorder_leaf;
-        a.preorder_sample = kd[i].preorder_sample;
-        b.preorder_leaf = kd[i].preorder_leaf + a.leaf_count;
-        b.preorder_sample = kd[i].preorder_sample + a.num_samples;
+        int leaves = 0, samples = 0;
+        for (int c = i, p = kd[i].parent; p >= 0; c = p, p = kd[p].parent)
+            if (kd[p].child1 == c)
+            {
+                const int a = kd[p].child0;
+                leaves += kd[a].leaf_count;
+                samples += kd[a].num_samples;
+            }
+        kd[i].preorder_leaf = leaves;
+        kd[i].preorder_sample = samples;
     }
 }
 
 // Entry points of the 32 build tasks and their sample / leaf bases
-// (Reconstruction.cpp:110-126, 132-143).
-__global__ void k_entry_points(const KdNode* kd, GridInfo* g, int num_kd)
+// (Reconstruction.cpp:110-126, 132-143), one lane per task.
+__global__ void __launch_bounds__(32) k_entry_points(const KdNode* kd, GridInfo* g, const int* level_count)
 {
-    int sb = 0, lb = 0;
-    for (int i = 0; i < 32; i++)
+    const int i = threadIdx.x;
+    int node = 0;
+    for (int j = 0; j < 5; j++)
     {
-        int node = 0;
-        for (int j = 0; j < 5; j++)
-        {
-            if (node == -1)
-                continue;
-            bool isLeaf = kd[node].child0 < 0;
-            if (i & (1 << j)) node = (!isLeaf) ? kd[node].child1 : -1;
-            else              node = (!isLeaf) ? kd[node].child0 : node;
-        }
-        g->entry[i] = node;
-        g->task_sample_base[i] = sb;
-        g->task_leaf_base[i] = lb;
-        if (node != -1)
-        {
-            sb += kd[node].num_samples;
-            lb += kd[node].leaf_count;
-        }
+        if (node == -1)
+            continue;
+        bool isLeaf = kd[node].child0 < 0;
+        if (i & (1 << j)) node = (!isLeaf) ? kd[node].child1 : -1;
+        else              node = (!isLeaf) ? kd[node].child0 : node;
     }
-    g->task_leaf_base[32] = lb;
-    g->num_kd = num_kd;
-    g->num_kd_leaves = lb;
-    g->num_accepted = sb;
+    const int ns = node != -1 ? kd[node].num_samples : 0, nl = node != -1 ? kd[node].leaf_count : 0;
+    int sb = ns, lb = nl;
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int x = __shfl_up_sync(0xffffffffu, sb, o), y = __shfl_up_sync(0xffffffffu, lb, o);
+        if (i >= o) { sb += x; lb += y; }
+    }
+    g->entry[i] = node;
+    g->task_sample_base[i] = sb - ns;
+    g->task_leaf_base[i] = lb - nl;
+    if (i == 31)
+    {
+        g->task_leaf_base[32] = lb;
+        g->num_kd = level_begin(level_count, kMaxKdLevels + 1);
+        g->num_kd_leaves = lb;
+        g->num_accepted = sb;
+    }
 }
 
 // Final sample offsets and build-task order of the kd leaves.  A node at depth
 // >= 5, or a leaf at depth < 5, belongs to the task given by its first five
 // child choices (its path bits).
-__global__ void k_kd_assign(KdNode* kd, int num_kd, const GridInfo* g, int* leaves_ordered)
+__global__ void k_kd_assign(KdNode* kd, const GridInfo* g, int* leaves_ordered)
 {
+    const int num_kd = g->num_kd;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < num_kd; i += gridDim.x * blockDim.x)
     {
         KdNode& nd = kd[i];
@@ -508,16 +529,57 @@ struct TWSortAccessor
     __device__ void swap(int a, int b) { int t = perm[a]; perm[a] = perm[b]; perm[b] = t; }
 };
 
-__global__ void k_leaf_prepare(const int* __restrict__ leaves_ordered, int num_leaves, const KdNode* __restrict__ kd,
-                               const int* __restrict__ cell_start, const int* __restrict__ cell_items, const GridInfo* g,
-                               const float4* __restrict__ rp_pos, const float4* __restrict__ rp_mot,
-                               const float4* __restrict__ rec, float W, float H, float c0, float c1,
-                               int* __restrict__ perm, float* __restrict__ box, Bounds* __restrict__ sbounds,
-                               float4* __restrict__ s_rec, float4* __restrict__ s_col,
-                               int* __restrict__ s_id, int* __restrict__ ordered_n, int* invalid_count)
+// A leaf's candidates in shared memory, one column per thread: (input index |
+// time code << 30, bits of w).  w > 0 and the times are 0, 1/2 and 1, so both
+// compare as integers.
+constexpr int kSortLeaf = 64;       // candidates of a leaf sorted in shared memory
+constexpr int kSortBlock = 64;
+struct TWColumn
 {
+    uint2 (*e)[kSortBlock];
+    int col;
+    __device__ int cmp(int a, int b) const
+    {
+        const uint2 x = e[a][col], y = e[b][col];
+        const unsigned tx = x.x >> 30, ty = y.x >> 30;
+        return tx != ty ? (tx < ty ? -1 : 1) : x.y < y.y ? -1 : x.y > y.y ? 1 : 0;
+    }
+    __device__ void swap(int a, int b) { const uint2 t = e[a][col]; e[a][col] = e[b][col]; e[b][col] = t; }
+};
+// fw_insertion_sort with the moving element in registers (the same permutation)
+__device__ __forceinline__ void fw_insertion_sort(TWColumn& a, int start, int size)
+{
+    for (int i = start + 1; i < start + size; i++)
+    {
+        const uint2 v = a.e[i][a.col];
+        const unsigned tv = v.x >> 30;
+        int j = i - 1;
+        for (; j >= start; j--)
+        {
+            const uint2 x = a.e[j][a.col];
+            const unsigned tx = x.x >> 30;
+            if (!(tx != tv ? tx > tv : x.y > v.y))
+                break;
+            a.e[j + 1][a.col] = x;
+        }
+        a.e[j + 1][a.col] = v;
+    }
+}
+
+// Candidates of every kd leaf in row-major cell order, sorted by (t, w) with
+// FW::sort (RTB.cpp:131-169), one thread per leaf.  The sort's chain of dependent
+// comparisons runs in shared memory; leaves of more than kSortLeaf candidates
+// (single cells) sort in place in global memory.  At 1280x720x8 this and
+// k_sample_prepare take 0.39 + 0.68 ms; one kernel that sorted in global memory
+// and bounded a leaf's samples one after another took 2.18 ms.
+__global__ void __launch_bounds__(kSortBlock)
+k_leaf_sort(const int* __restrict__ leaves_ordered, int num_leaves, const KdNode* __restrict__ kd,
+            const int* __restrict__ cell_start, const int* __restrict__ cell_items, const GridInfo* g,
+            const float4* __restrict__ rp_pos, int* __restrict__ perm, int* __restrict__ ordered_n,
+            int* __restrict__ leaf_of, bool wide_ids)
+{
+    __shared__ uint2 sh[kSortLeaf][kSortBlock];
     const int gw = g->gw;
-    int invalid = 0;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < num_leaves; r += gridDim.x * blockDim.x)
     {
         const KdNode nd = kd[leaves_ordered[r]];
@@ -526,66 +588,89 @@ __global__ void k_leaf_prepare(const int* __restrict__ leaves_ordered, int num_l
         if (n == 0)
             continue;
         const int off = nd.sample_offset;
-        int k = 0;
-        for (int y = nd.y0; y < nd.y1; y++)
-            for (int x = nd.x0; x < nd.x1; x++)
-            {
-                int c = y * gw + x;
-                for (int q = cell_start[c]; q < cell_start[c + 1]; q++)
-                    perm[off + k++] = cell_items[q];
-            }
-        TWSortAccessor acc{ perm + off, rp_pos };
-        fw_sort(acc, 0, n);
         for (int j = 0; j < n; j++)
+            leaf_of[off + j] = r;
+        int k = 0;
+        // the cells of a grid row are neighbours in the buckets
+        if (n > kSortLeaf || wide_ids)
         {
-            const int id = perm[off + j];
-            const float4 p = rp_pos[id];
-            const float4 m = rp_mot[id];
-            const float sx = p.x, sy = p.y, sw = p.z, st = p.w;
-            const float mv[3] = { m.x, m.y, m.z };
-            float xywt0[3] = { sx * sw - mv[0] * st, sy * sw - mv[1] * st, sw - mv[2] * st };
-            Bounds b;
-            tux_planes(xywt0, mv, W, H, c0, c1, b);
-            sbounds[off + j] = b;
-            float* bx = box + (size_t)(off + j) * 8;
-            if (bounds_valid(b))
-            {
-                float ta = b.tspan[0], tb = b.tspan[1];
-                float base[3] = { sx * sw, sy * sw, sw };
-                float xa[3], xb[3];
-                for (int q = 0; q < 3; q++)
-                {
-                    xa[q] = base[q] + mv[q] * (ta - st);
-                    xb[q] = base[q] + mv[q] * (tb - st);
-                }
-                float ca = rcp(xa[2]), cb = rcp(xb[2]);
-                float xyta[2] = { xa[0] * ca, xa[1] * ca };
-                float xytb[2] = { xb[0] * cb, xb[1] * cb };
-                float oodt = 1.0f / (tb - ta);
-                float dxdt = (xytb[0] - xyta[0]) * oodt;
-                float dydt = (xytb[1] - xyta[1]) * oodt;
-                float xyt0[2] = { xyta[0] - dxdt * ta, xyta[1] - dydt * ta };
-                float xyt1[2] = { xytb[0] + dxdt * (1.0f - tb), xytb[1] + dydt * (1.0f - tb) };
-                float cocta = c0 / xa[2] + c1;
-                float coctb = c0 / xb[2] + c1;
-                bx[0] = xyt0[0] + cocta; bx[1] = xyt0[1] + cocta;
-                bx[2] = xyt0[0] - cocta; bx[3] = xyt0[1] - cocta;
-                bx[4] = xyt1[0] + coctb; bx[5] = xyt1[1] + coctb;
-                bx[6] = xyt1[0] - coctb; bx[7] = xyt1[1] - coctb;
-            }
-            else
-                invalid++;
-            // tree-ordered sample record (Reconstruction.hpp:73-86 Sample, color alpha 1)
-            float4 r1 = __ldg(&rec[(size_t)id * 4 + 1]);
-            float4 r2 = __ldg(&rec[(size_t)id * 4 + 2]);
-            s_rec[2 * (off + j)] = p;
-            s_rec[2 * (off + j) + 1] = make_float4(mv[0], mv[1], mv[2], c0 / sw + c1);
-            s_col[off + j] = make_float4(r1.w, r2.x, r2.y, 1.0f);
-            s_id[off + j] = id;
+            for (int y = nd.y0; y < nd.y1; y++)
+                for (int q = cell_start[y * gw + nd.x0]; q < cell_start[y * gw + nd.x1]; q++)
+                    perm[off + k++] = cell_items[q];
+            TWSortAccessor acc{ perm + off, rp_pos };
+            fw_sort(acc, 0, n);
+            continue;
         }
+        for (int y = nd.y0; y < nd.y1; y++)
+            for (int q = cell_start[y * gw + nd.x0]; q < cell_start[y * gw + nd.x1]; q++)
+            {
+                const int id = cell_items[q];
+                const float4 p = rp_pos[id];
+                sh[k++][threadIdx.x] = make_uint2((unsigned)id | (unsigned)(2.0f * p.w) << 30, __float_as_uint(p.z));
+            }
+        TWColumn col{ sh, (int)threadIdx.x };
+        if (n < 16)
+            fw_insertion_sort(col, 0, n);
+        else
+            fw_sort(col, 0, n);
+        for (int j = 0; j < n; j++)
+            perm[off + j] = (int)(sh[j][threadIdx.x].x & 0x3fffffffu);
     }
-    if (invalid)
-        atomicAdd(invalid_count, invalid);
+}
+
+// Bounds and t=0/t=1 boxes of every candidate (RTB.cpp:170-213) and its
+// tree-ordered record, one thread per sample slot.
+__global__ void k_sample_prepare(const int* __restrict__ perm, int num_slots, const float4* __restrict__ rp_pos,
+                                 const float4* __restrict__ rp_mot, const float4* __restrict__ rec, float W, float H,
+                                 float c0, float c1, float* __restrict__ box, Bounds* __restrict__ sbounds,
+                                 float4* __restrict__ s_rec, float4* __restrict__ s_col, int* __restrict__ s_id,
+                                 int* __restrict__ invalid, int* invalid_count)
+{
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < num_slots; j += gridDim.x * blockDim.x)
+    {
+        const int id = perm[j];
+        const float4 p = rp_pos[id];
+        const float4 m = rp_mot[id];
+        const float sx = p.x, sy = p.y, sw = p.z, st = p.w;
+        const float mv[3] = { m.x, m.y, m.z };
+        float xywt0[3] = { sx * sw - mv[0] * st, sy * sw - mv[1] * st, sw - mv[2] * st };
+        Bounds b;
+        tux_planes(xywt0, mv, W, H, c0, c1, b);
+        sbounds[j] = b;
+        if (bounds_valid(b))
+        {
+            float ta = b.tspan[0], tb = b.tspan[1];
+            float base[3] = { sx * sw, sy * sw, sw };
+            float xa[3], xb[3];
+            for (int q = 0; q < 3; q++)
+            {
+                xa[q] = base[q] + mv[q] * (ta - st);
+                xb[q] = base[q] + mv[q] * (tb - st);
+            }
+            float ca = rcp(xa[2]), cb = rcp(xb[2]);
+            float xyta[2] = { xa[0] * ca, xa[1] * ca };
+            float xytb[2] = { xb[0] * cb, xb[1] * cb };
+            float oodt = 1.0f / (tb - ta);
+            float dxdt = (xytb[0] - xyta[0]) * oodt;
+            float dydt = (xytb[1] - xyta[1]) * oodt;
+            float xyt0[2] = { xyta[0] - dxdt * ta, xyta[1] - dydt * ta };
+            float xyt1[2] = { xytb[0] + dxdt * (1.0f - tb), xytb[1] + dydt * (1.0f - tb) };
+            float cocta = c0 / xa[2] + c1;
+            float coctb = c0 / xb[2] + c1;
+            float4* bx = reinterpret_cast<float4*>(box) + 2 * (size_t)j;
+            bx[0] = make_float4(xyt0[0] + cocta, xyt0[1] + cocta, xyt0[0] - cocta, xyt0[1] - cocta);
+            bx[1] = make_float4(xyt1[0] + coctb, xyt1[1] + coctb, xyt1[0] - coctb, xyt1[1] - coctb);
+        }
+        else
+            invalid[atomicAdd(invalid_count, 1)] = j;
+        // tree-ordered sample record (Reconstruction.hpp:73-86 Sample, color alpha 1)
+        const float4 r1 = __ldg(&rec[(size_t)id * 4 + 1]);
+        const float4 r2 = __ldg(&rec[(size_t)id * 4 + 2]);
+        s_rec[2 * (size_t)j] = p;
+        s_rec[2 * (size_t)j + 1] = make_float4(mv[0], mv[1], mv[2], c0 / sw + c1);
+        s_col[j] = make_float4(r1.w, r2.x, r2.y, 1.0f);
+        s_id[j] = id;
+    }
 }
 
 // Per build task: exclusive running maximum of the candidate counts and the
@@ -644,51 +729,49 @@ __device__ __forceinline__ int alloc_round(int m)
 // Candidates with invalid bounds take the boxes the reused per-task arrays hold
 // at their index: the value written there by the most recent earlier leaf of the
 // task, unless a reallocation in between cleared it (elements at or beyond the
-// previous size are zero after Array::realloc).
+// previous size are zero after Array::realloc).  One thread per such candidate
+// (1280x720x8: 0.06 ms; one thread per leaf took 0.53 ms).
 __global__ void k_stale_boxes(const int* __restrict__ leaves_ordered, const GridInfo* g, const KdNode* __restrict__ kd,
                               const int* __restrict__ ordered_n, const int* __restrict__ prefmax,
                               const int* __restrict__ prevn, const Bounds* __restrict__ sbounds,
-                              float* __restrict__ box, int num_leaves, int task_of_first)
+                              float* __restrict__ box, const int* __restrict__ leaf_of,
+                              const int* __restrict__ invalid, const int* __restrict__ num_invalid)
 {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < num_leaves; r += gridDim.x * blockDim.x)
+    const int total = *num_invalid;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x)
     {
-        const int n = ordered_n[r];
-        if (n == 0)
-            continue;
-        const KdNode nd = kd[leaves_ordered[r]];
-        const int off = nd.sample_offset;
+        const int slot = invalid[q], r = leaf_of[slot];
+        const int i = slot - kd[leaves_ordered[r]].sample_offset;
         // task of this ordered rank
         int t = 0;
         while (t < 31 && g->task_leaf_base[t + 1] <= r) t++;
         const int tb = g->task_leaf_base[t];
-        for (int i = 0; i < n; i++)
+        float4 v0 = make_float4(0, 0, 0, 0), v1 = v0;
+        // state after this leaf's resize
+        bool realloc_here = ordered_n[r] > alloc_round(prefmax[r]);
+        if (!(realloc_here && i >= prevn[r]))
         {
-            if (bounds_valid(sbounds[off + i]))
-                continue;
-            float v[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-            // state after this leaf's resize
-            bool realloc_here = n > alloc_round(prefmax[r]);
-            if (!(realloc_here && i >= prevn[r]))
+            for (int k = r - 1; k >= tb; k--)
             {
-                for (int k = r - 1; k >= tb; k--)
+                const int nk = ordered_n[k];
+                if (nk == 0)
+                    continue;
+                const int offk = kd[leaves_ordered[k]].sample_offset;
+                if (nk > i && bounds_valid(sbounds[offk + i]))
                 {
-                    const int nk = ordered_n[k];
-                    if (nk == 0)
-                        continue;
-                    const int offk = kd[leaves_ordered[k]].sample_offset;
-                    if (nk > i && bounds_valid(sbounds[offk + i]))
-                    {
-                        for (int q = 0; q < 8; q++) v[q] = box[(size_t)(offk + i) * 8 + q];
-                        break;
-                    }
-                    if (nk > alloc_round(prefmax[k]) && i >= prevn[k])
-                        break;      // cleared by the reallocation at leaf k
+                    const float4* b = reinterpret_cast<const float4*>(box) + 2 * (size_t)(offk + i);
+                    v0 = b[0];
+                    v1 = b[1];
+                    break;
                 }
+                if (nk > alloc_round(prefmax[k]) && i >= prevn[k])
+                    break;      // cleared by the reallocation at leaf k
             }
-            for (int q = 0; q < 8; q++) box[(size_t)(off + i) * 8 + q] = v[q];
         }
+        float4* b = reinterpret_cast<float4*>(box) + 2 * (size_t)slot;
+        b[0] = v0;
+        b[1] = v1;
     }
-    (void)task_of_first;
 }
 
 __device__ __forceinline__ void bnode_from_bounds(BNode& n, const Bounds& b)
@@ -870,118 +953,192 @@ __device__ __forceinline__ void store_node(QNode* nodes, float2* tspans, int slo
     tspans[slot] = make_float2(n.tspan[0], n.tspan[1]);
 }
 
+// By a group of G neighbouring lanes: the pairs' costs in parallel, the first
+// cheapest pair in the reference's order (i, then j).
+template <int G>
 __device__ int emit_nodes(bool is_root, BNode* f, int size, QNode* nodes, float2* tspans, int* node_counter)
 {
+    const int lane = threadIdx.x & (G - 1);
+    const unsigned group = (G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (threadIdx.x & 31 & ~(G - 1)));
     const int lim = is_root ? 1 : 4;
-    // node costs of the frontier entries (recomputed per step as the reference does)
     while (size > lim)
     {
-        float minCost = kF32Max;
-        int mi = -1, mj = -1;
-        for (int i = 0; i < size; i++)
+        float best = kF32Max;
+        unsigned at = 0xffffffffu;      // i << 16 | j
+        for (int p = lane, i = 0, row = 0;; p += G)
         {
-            const BNode n0 = f[i];
-            const float c0 = bnode_cost(n0);
-            for (int j = i + 1; j < size; j++)
+            // pair p: rows of i against j > i; row = pairs before row i
+            while (i < size - 1 && p >= row + size - 1 - i)
             {
-                const BNode n1 = f[j];
-                BNode m;
-                node_merge(n0, n1, m);
-                float cost = bnode_cost(m) - (c0 + bnode_cost(n1));
-                if (cost < minCost)
-                {
-                    minCost = cost;
-                    mi = i; mj = j;
-                }
+                row += size - 1 - i;
+                i++;
+            }
+            if (i >= size - 1)
+                break;
+            const int j = i + 1 + (p - row);
+            const BNode n0 = f[i], n1 = f[j];
+            BNode m;
+            node_merge(n0, n1, m);
+            const float cost = bnode_cost(m) - (bnode_cost(n0) + bnode_cost(n1));
+            if (cost < best)
+            {
+                best = cost;
+                at = (unsigned)i << 16 | (unsigned)j;
             }
         }
-        if (mi < 0) { mi = 0; mj = 1; }
-        const BNode n0 = f[mi], n1 = f[mj];
-        BNode m;
-        node_merge(n0, n1, m);
-        int slot = atomicAdd(node_counter, 2);
-        store_node(nodes, tspans, slot, n0);
-        store_node(nodes, tspans, slot + 1, n1);
-        m.ref = slot;
-        f[mi] = m;
-        f[mj] = f[size - 1];
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1)
+        {
+            const float ob = __shfl_xor_sync(group, best, o);
+            const unsigned oa = __shfl_xor_sync(group, at, o);
+            if (ob < best || (ob == best && oa < at))
+            {
+                best = ob;
+                at = oa;
+            }
+        }
+        const int mi = at == 0xffffffffu ? 0 : (int)(at >> 16), mj = at == 0xffffffffu ? 1 : (int)(at & 0xffffu);
+        if (lane == 0)
+        {
+            const BNode n0 = f[mi], n1 = f[mj];
+            BNode m;
+            node_merge(n0, n1, m);
+            int slot = atomicAdd(node_counter, 2);
+            store_node(nodes, tspans, slot, n0);
+            store_node(nodes, tspans, slot + 1, n1);
+            m.ref = slot;
+            f[mi] = m;
+            f[mj] = f[size - 1];
+        }
+        __syncwarp(group);
         size--;
     }
     return size;
 }
 
-__global__ void k_emit_level(KdNode* kd, const int* levels, int L, BNode* pending, QNode* nodes, float2* tspans,
+// A group of kEmitGroup lanes per kd node of level L.  A level above the lowest
+// ones holds few nodes, so its time is one node's chain of merges: up to 74 of
+// them for eight frontier nodes, 15 with eight lanes (1280x720x8, 17 levels:
+// 0.95 ms against 2.85 with one thread per node).
+constexpr int kEmitGroup = 8;
+__global__ void k_emit_level(KdNode* kd, const int* level_count, int L, BNode* pending, QNode* nodes, float2* tspans,
                              int* node_counter)
 {
-    const int lo = levels[2 * L], hi = levels[2 * L + 1];
-    for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
+    const int lo = level_begin(level_count, L), hi = lo + level_count[L];
+    const int lane = threadIdx.x & (kEmitGroup - 1);
+    const unsigned group = ((1u << kEmitGroup) - 1u) << (threadIdx.x & 31 & ~(kEmitGroup - 1));
+    const int stride = gridDim.x * blockDim.x / kEmitGroup;
+    for (int i = lo + (blockIdx.x * blockDim.x + threadIdx.x) / kEmitGroup; i < hi; i += stride)
     {
         const KdNode nd = kd[i];
         if (nd.child0 < 0 || nd.depth < 5)
             continue;
-        const KdNode a = kd[nd.child0], b = kd[nd.child1];
-        const int off = nd.sample_offset;
-        const int fa = a.frontier, fb = b.frontier;
-        // child0's frontier is at [off, off+fa); bring child1's next to it
-        BNode* f = pending + off;
-        const BNode* src = pending + b.sample_offset;
-        for (int q = 0; q < fb; q++)
-            f[fa + q] = src[q];
-        int size = emit_nodes(false, f, fa + fb, nodes, tspans, node_counter);
-        kd[i].frontier = size;
+        const int fa = kd[nd.child0].frontier, fb = kd[nd.child1].frontier;
+        // child0's frontier is at [off, off+fa); bring child1's next to it (it
+        // moves down, kEmitGroup nodes at a time)
+        BNode* f = pending + nd.sample_offset;
+        const BNode* src = pending + kd[nd.child1].sample_offset;
+        for (int q = 0; q < fb; q += kEmitGroup)
+        {
+            BNode t;
+            if (q + lane < fb)
+                t = src[q + lane];
+            __syncwarp(group);
+            if (q + lane < fb)
+                f[fa + q + lane] = t;
+            __syncwarp(group);
+        }
+        const int size = emit_nodes<kEmitGroup>(false, f, fa + fb, nodes, tspans, node_counter);
+        if (lane == 0)
+            kd[i].frontier = size;
     }
 }
 
-// Serial top of the tree (Reconstruction.cpp:192-203) and the root.
-__global__ void k_top(KdNode* kd, GridInfo* g, BNode* pending, BNode* top, QNode* nodes, float2* tspans,
-                      int* node_counter)
+// Top of the tree (Reconstruction.cpp:192-203) and the root: the tasks'
+// frontiers merged in pairs, level by level, one warp per pair (0.06 ms; one
+// thread took 0.90 ms).
+__global__ void __launch_bounds__(512)
+k_top(KdNode* kd, GridInfo* g, BNode* pending, BNode* top, QNode* nodes, float2* tspans, int* node_counter)
 {
-    int start[32], count[32];
-    int used = 0;
-    for (int i = 0; i < 32; i++)
+    __shared__ int start[32], count[32], dst[16];
+    __shared__ int used;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0)
     {
-        start[i] = used;
-        count[i] = 0;
-        int e = g->entry[i];
-        if (e < 0)
-            continue;
-        const KdNode nd = kd[e];
-        int fs = nd.frontier;
-        if (used + fs > kTopCap) { g->error = kErrTopCap; return; }
-        for (int q = 0; q < fs; q++)
-            top[used + q] = pending[nd.sample_offset + q];
-        count[i] = fs;
-        used += fs;
+        const int e = g->entry[lane];
+        const int fs = e < 0 ? 0 : kd[e].frontier;
+        int sum = fs;
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int x = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += x;
+        }
+        start[lane] = sum - fs;
+        count[lane] = fs;
+        if (lane == 31)
+            used = sum;
     }
+    __syncthreads();
+    if (used > kTopCap)
+    {
+        if (threadIdx.x == 0) g->error = kErrTopCap;
+        return;
+    }
+    for (int i = warp; i < 32; i += 16)
+    {
+        const int e = g->entry[i];
+        for (int q = lane; q < count[i]; q += 32)
+            top[start[i] + q] = pending[kd[e].sample_offset + q];
+    }
+    __syncthreads();
     for (int j = 0; j < 5; j++)
     {
-        int offset = 1 << j;
-        for (int i = 0; i < 32; i += 2 * offset)
+        const int offset = 1 << j, pairs = 16 >> j;
+        if (threadIdx.x == 0)
+            for (int p = 0; p < pairs; p++)
+            {
+                dst[p] = used;
+                used += count[2 * offset * p] + count[2 * offset * p + offset];
+            }
+        __syncthreads();
+        if (used > kTopCap)
         {
-            int na = count[i], nb = count[i + offset];
-            if (used + na + nb > kTopCap) { g->error = kErrTopCap; return; }
-            int s = used;
-            for (int q = 0; q < na; q++) top[s + q] = top[start[i] + q];
-            for (int q = 0; q < nb; q++) top[s + na + q] = top[start[i + offset] + q];
-            used += na + nb;
-            int size = emit_nodes(j == 4, top + s, na + nb, nodes, tspans, node_counter);
-            start[i] = s;
-            count[i] = size;
+            if (threadIdx.x == 0) g->error = kErrTopCap;
+            return;
         }
+        if (warp < pairs)
+        {
+            const int i = 2 * offset * warp, s = dst[warp];
+            const int na = count[i], nb = count[i + offset];
+            for (int q = lane; q < na; q += 32) top[s + q] = top[start[i] + q];
+            for (int q = lane; q < nb; q += 32) top[s + na + q] = top[start[i + offset] + q];
+            __syncwarp();
+            const int size = emit_nodes<32>(j == 4, top + s, na + nb, nodes, tspans, node_counter);
+            __syncwarp();
+            if (lane == 0)
+            {
+                start[i] = s;
+                count[i] = size;
+            }
+        }
+        __syncthreads();
     }
-    if (count[0] == 1)
+    if (threadIdx.x == 0)
     {
-        int slot = atomicAdd(node_counter, 1);
-        store_node(nodes, tspans, slot, top[start[0]]);
-        g->root = slot;
-        g->height = top[start[0]].height;
+        if (count[0] == 1)
+        {
+            int slot = atomicAdd(node_counter, 1);
+            store_node(nodes, tspans, slot, top[start[0]]);
+            g->root = slot;
+            g->height = top[start[0]].height;
+        }
+        else
+        {
+            g->root = -1;
+            g->height = 0;
+        }
+        g->num_nodes = *node_counter;
     }
-    else
-    {
-        g->root = -1;
-        g->height = 0;
-    }
-    g->num_nodes = *node_counter;
 }
 
 int grid_for(const Ctx& c, size_t n, int block)
@@ -1056,9 +1213,9 @@ tlfr_status build_hierarchy(Ctx& c, const float* d_records)
     if (!c.d_grid)
         CK(cudaMalloc(&c.d_grid, sizeof(GridInfo) + sizeof(GridAccum) + 64 * sizeof(int)));
     if (!c.kd_level)
-        CK(cudaMalloc(&c.kd_level, sizeof(int) * 2 * (kMaxKdLevels + 2)));
+        CK(cudaMalloc(&c.kd_level, sizeof(int) * (kMaxKdLevels + 2)));
     GridAccum* acc = reinterpret_cast<GridAccum*>(reinterpret_cast<char*>(c.d_grid) + sizeof(GridInfo));
-    int* counters = reinterpret_cast<int*>(acc + 1);    // [0] kd counter, [1] node counter, [2] invalid, [3] scan total
+    int* counters = reinterpret_cast<int*>(acc + 1);    // [1] node counter, [2] invalid, [3] scan total
 
     // --- reprojection, bounding box, hit histogram ---
     CK(cudaMemsetAsync(c.hits, 0, sizeof(int) * (size_t)c.W * c.H, s));
@@ -1119,31 +1276,27 @@ tlfr_status build_hierarchy(Ctx& c, const float* d_records)
         CK(cudaMalloc(&c.kd_leaves_ordered, sizeof(int) * kd_max));
         c.kd_cap = kd_max;
     }
-    TLFR_LAUNCH(c, k_kd_init, 1, 1, s, c.kd, c.kd_level, c.d_grid, counters + 0);
-    for (int L = 0; L < kMaxKdLevels; L++)
+    // a cell range halves at every split, so the levels follow from the grid
+    int levels = 1;
+    for (int w = 1; w < c.grid.gw; w <<= 1) levels++;
+    for (int h = 1; h < c.grid.gh; h <<= 1) levels++;
+    if (levels > kMaxKdLevels)
     {
-        TLFR_LAUNCH(c, k_kd_level, c.num_sms * 4, 256, s, c.kd, c.kd_level, L, c.cell_start, c.d_grid, counters + 0);
-        TLFR_LAUNCH(c, k_kd_next, 1, 1, s, c.kd_level, L, counters + 0, c.d_grid);
+        c.error = "kd split deeper than supported";
+        return TLFR_OVERFLOW;
     }
-    for (int L = kMaxKdLevels - 1; L >= 0; L--)
-        TLFR_LAUNCH(c, k_kd_up, c.num_sms * 4, 256, s, c.kd, c.kd_level, L);
-    for (int L = 0; L < kMaxKdLevels; L++)
-        TLFR_LAUNCH(c, k_kd_down, c.num_sms * 4, 256, s, c.kd, c.kd_level, L);
+    TLFR_LAUNCH(c, k_kd_init, 1, 64, s, c.kd, c.kd_level, c.d_grid);
+    for (int L = 0; L < levels; L++)
+    {
+        const size_t most = std::min<size_t>((size_t)1 << std::min(L, 30), ncell);
+        TLFR_LAUNCH(c, k_kd_level, std::min(c.num_sms * 4, grid_for(c, most, 256)), 256, s, c.kd, c.kd_level, L,
+                    c.cell_start, c.d_grid);
+    }
+    TLFR_LAUNCH(c, k_kd_up, grid_for(c, 2 * ncell, 256), 256, s, c.kd, c.kd_level);
+    TLFR_LAUNCH(c, k_kd_offsets, grid_for(c, 2 * ncell, 256), 256, s, c.kd, c.kd_level);
+    TLFR_LAUNCH(c, k_entry_points, 1, 32, s, c.kd, c.d_grid, c.kd_level);
+    TLFR_LAUNCH(c, k_kd_assign, grid_for(c, 2 * ncell, 256), 256, s, c.kd, c.d_grid, c.kd_leaves_ordered);
     CK(cudaGetLastError());
-    int num_kd = 0;
-    CK(cudaMemcpyAsync(&num_kd, counters + 0, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    {
-        int last[2];
-        CK(cudaMemcpy(last, c.kd_level + 2 * kMaxKdLevels, sizeof(int) * 2, cudaMemcpyDeviceToHost));
-        if (last[1] != last[0])
-        {
-            c.error = "kd split deeper than supported";
-            return TLFR_OVERFLOW;
-        }
-    }
-    TLFR_LAUNCH(c, k_entry_points, 1, 1, s, c.kd, c.d_grid, num_kd);
-    TLFR_LAUNCH(c, k_kd_assign, grid_for(c, num_kd, 256), 256, s, c.kd, num_kd, c.d_grid, c.kd_leaves_ordered);
     CK(cudaMemcpyAsync(&c.grid, c.d_grid, sizeof(GridInfo), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     const int num_leaves = c.grid.num_kd_leaves;
@@ -1187,22 +1340,28 @@ tlfr_status build_hierarchy(Ctx& c, const float* d_records)
     }
 
     // --- leaves ---
-    TLFR_LAUNCH(c, k_leaf_prepare, grid_for(c, num_leaves, 128), 128, s, 
-        c.kd_leaves_ordered, num_leaves, c.kd, c.cell_start, c.cell_items, c.d_grid, c.rp_pos, c.rp_mot, rec,
-        (float)c.W, (float)c.H, c.coc[0], c.coc[1], c.perm, c.box, c.sbounds, c.s_rec, c.s_col, c.s_id,
-        c.ordered_n, counters + 2);
+    // until the surface scan, c.surface holds each slot's leaf and c.pending the list of slots with invalid bounds
+    int* invalid = reinterpret_cast<int*>(c.pending);
+    TLFR_LAUNCH(c, k_leaf_sort, grid_for(c, num_leaves, kSortBlock), kSortBlock, s, c.kd_leaves_ordered, num_leaves, c.kd,
+                c.cell_start, c.cell_items, c.d_grid, c.rp_pos, c.perm, c.ordered_n, c.surface, n >= ((size_t)1 << 30));
+    TLFR_LAUNCH(c, k_sample_prepare, grid_for(c, nacc, 128), 128, s, c.perm, (int)nacc, c.rp_pos, c.rp_mot, rec,
+                (float)c.W, (float)c.H, c.coc[0], c.coc[1], c.box, c.sbounds, c.s_rec, c.s_col, c.s_id, invalid,
+                counters + 2);
     TLFR_LAUNCH(c, k_task_prefix, 32, 1024, s, c.d_grid, c.ordered_n, c.ordered_prefmax, c.leaf_task_rank);
-    TLFR_LAUNCH(c, k_stale_boxes, grid_for(c, num_leaves, 128), 128, s, c.kd_leaves_ordered, c.d_grid, c.kd, c.ordered_n,
-                                                            c.ordered_prefmax, c.leaf_task_rank, c.sbounds, c.box,
-                                                            num_leaves, 0);
+    TLFR_LAUNCH(c, k_stale_boxes, grid_for(c, nacc, 128), 128, s, c.kd_leaves_ordered, c.d_grid, c.kd, c.ordered_n,
+                c.ordered_prefmax, c.leaf_task_rank, c.sbounds, c.box, c.surface, invalid, counters + 2);
     TLFR_LAUNCH(c, k_leaf_scan, grid_for(c, num_leaves, 128), 128, s, c.kd_leaves_ordered, num_leaves, c.kd, c.s_rec, c.box,
                                                           c.sbounds, c.surface, c.pending);
     CK(cudaGetLastError());
 
     // --- emitNodes bottom-up, then the serial top ---
-    for (int L = c.grid.kd_levels; L >= 5; L--)
-        TLFR_LAUNCH(c, k_emit_level, c.num_sms * 4, 128, s, c.kd, c.kd_level, L, c.pending, c.nodes, c.node_tspan, counters + 1);
-    TLFR_LAUNCH(c, k_top, 1, 1, s, c.kd, c.d_grid, c.pending, c.top, c.nodes, c.node_tspan, counters + 1);
+    for (int L = levels - 1; L >= 5; L--)
+    {
+        const size_t most = std::min<size_t>((size_t)1 << std::min(L, 30), (size_t)c.grid.num_kd) * kEmitGroup;
+        TLFR_LAUNCH(c, k_emit_level, grid_for(c, most, 128), 128, s, c.kd, c.kd_level, L, c.pending, c.nodes,
+                    c.node_tspan, counters + 1);
+    }
+    TLFR_LAUNCH(c, k_top, 1, 512, s, c.kd, c.d_grid, c.pending, c.top, c.nodes, c.node_tspan, counters + 1);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&c.grid, c.d_grid, sizeof(GridInfo), cudaMemcpyDeviceToHost, s));
     int inv = 0;

@@ -57,7 +57,7 @@ struct __align__(16) KdNode
     int preorder_sample;    // sample offset of the subtree in preorder
     int sample_offset;      // final sample offset (task order, as the reference lays samples out)
     int frontier;           // size of the subtree's frontier after emitNodes
-    int pad;
+    int arrived;            // children whose counts are in (k_kd_up)
 };
 
 // Scalars computed on the device during the build.
@@ -80,7 +80,6 @@ struct GridInfo
     int   task_leaf_base[33];
     int   num_invalid;          // samples with invalid bounds
     int   error;                // nonzero: build capacity error code
-    int   kd_levels;
 };
 
 // Per-reconstruction device counters (TreeGather::Stats, Reconstruction.hpp:134-147).
@@ -127,7 +126,7 @@ struct Ctx
 
     // kd tree
     KdNode* kd = nullptr;
-    int*    kd_level = nullptr;     // level ranges: [2*L], [2*L+1]
+    int*    kd_level = nullptr;     // nodes per level
     int*    kd_leaves_ordered = nullptr;   // kd leaf ids in build-task order
     size_t  kd_cap = 0;
 
