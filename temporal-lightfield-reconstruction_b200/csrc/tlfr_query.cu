@@ -1037,6 +1037,17 @@ __device__ __forceinline__ Query query_of(const QParams& P, long long q)
     return make_query(P, (int)(pix % P.W), (int)(pix / P.W), i);
 }
 
+// Entries of a queue of n that a warp takes at a time: at most 32, and so few
+// that the last round of nwarps warps is nearly full (a warp works on its
+// entries one after another, so a short queue wants few per warp: the full path
+// of 4.5 K entries at 64x48x4 0.10 ms against 0.30 with 32 each, the retry tier
+// of 57 K at one sample per pixel of 1280x720x8 0.46 ms against 0.65).
+__device__ __forceinline__ int entries_per_warp(long long n, int nwarps)
+{
+    const long long rounds = (n + 32LL * nwarps - 1) / (32LL * nwarps);
+    return rounds == 0 ? 32 : (int)((n + rounds * nwarps - 1) / (rounds * nwarps));
+}
+
 // Append value to a queue when pred holds, one atomic per warp.  All 32 lanes
 // of the warp must call it.
 __device__ __forceinline__ void warp_append(int* queue, int* count, bool pred, int value)
@@ -1087,10 +1098,13 @@ enum { kLightPlain = 0, kLightFirst = 1, kLightRetry = 2 };
 //     nodes a warp reaches is then 3.8x one output sample's at 1920x1080x8
 //     (5.3x for a pixel's 32 consecutive samples); batches choose the shape
 //     per frame by timing (autotuner).
-//   kMapLinear: q = block iteration * 128 + thread (the pinhole image's one
-//     sample per pixel, and M not a multiple of 4*sw).
+//   kMapSingle: a warp takes one output sample of each pixel of an 8x4 tile, its
+//     block four such units in turn over samples, then tiles (M not a multiple of
+//     4*sw, so the pinhole image's one sample per pixel: first tier at 1280x720x8
+//     1.97 ms against 2.12 with 32 consecutive pixels of a row).
+//   kMapLinear: q = block iteration * 128 + thread (the router's coarse pass).
 // Output sample ids q = pixel * M + i are unchanged (qcol, queues).
-enum { kMapLinear = 0, kMapTiles = 1 };
+enum { kMapLinear = 0, kMapTiles = 1, kMapSingle = 2 };
 
 struct LightMap
 {
@@ -1114,6 +1128,15 @@ __device__ __forceinline__ bool light_query_id(const QParams& P, const LightMap&
         q = u * kBlock + t;
         return q < num_queries;
     }
+    if (L.mode == kMapSingle)
+    {
+        const long long w = u * 4 + (t >> 5), tile = w / P.M;
+        const int l = t & 31, i = (int)(w - tile * P.M);
+        const int x = (int)(tile % L.tiles_x) * 8 + (l & 7);
+        const long long y = tile / L.tiles_x * 4 + (l >> 3);
+        q = (y * P.W + x) * P.M + i;
+        return x < P.W && y < P.H;
+    }
     const long long tile = u / L.groups;
     const int g = (int)(u - tile * L.groups);
     const int px = L.tw * L.th;
@@ -1127,9 +1150,9 @@ __device__ __forceinline__ bool light_query_id(const QParams& P, const LightMap&
 
 // One block iteration u of the light pass (RO.cpp:94-99, 165-304 for the common
 // case): each lane collects its own output sample's leaves at 1R, then the warp
-// scans the output samples in turn.  kLightRetry: the output samples are
-// retry[u * kBlock + thread] for indices below num_queries; kLightFirst: those
-// that outgrow the capacities are appended to retry.
+// scans the output samples in turn.  kLightRetry: warp w of the iterations takes
+// per_warp output samples from retry[w * per_warp] on, of num_queries in all;
+// kLightFirst: those that outgrow the capacities are appended to retry.
 //
 // A sample settles when the 1R fetch ends with exactly one surface, or when the
 // first surface holds samples in all four quadrants by the time a second one
@@ -1161,7 +1184,8 @@ template <bool PROBE, int LEAF, int STACK, int MODE>
 __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, long long u, long long num_queries,
                                            float4* __restrict__ qcol, int* __restrict__ heavy,
                                            int* __restrict__ heavy_count, LightShared<LEAF, STACK>& S,
-                                           int* __restrict__ retry = nullptr, int* __restrict__ retry_count = nullptr)
+                                           int* __restrict__ retry = nullptr, int* __restrict__ retry_count = nullptr,
+                                           int per_warp = 32)
 {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u, upto = (2u << lane) - 1u;
@@ -1171,8 +1195,8 @@ __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, 
     bool valid;
     if (MODE == kLightRetry)
     {
-        const long long k = u * kBlock + threadIdx.x;
-        valid = k < num_queries;
+        const long long k = (u * (kBlock / 32) + (threadIdx.x >> 5)) * per_warp + lane;
+        valid = lane < per_warp && k < num_queries;
         q = valid ? retry[k] : 0;
     }
     else
@@ -1508,8 +1532,9 @@ k_query_light(QParams P, LightMap L, long long num_queries, float4* __restrict__
     if (MODE == kLightRetry)
     {
         const long long n = *retry_count;
-        for (long long u = blockIdx.x; u * kBlock < n; u += gridDim.x)
-            light_unit<PROBE, LEAF, STACK, MODE>(P, L, u, n, qcol, heavy, heavy_count, sh, retry);
+        const int per = entries_per_warp(n, gridDim.x * (kBlock / 32));
+        for (long long u = blockIdx.x; u * (kBlock / 32) * per < n; u += gridDim.x)
+            light_unit<PROBE, LEAF, STACK, MODE>(P, L, u, n, qcol, heavy, heavy_count, sh, retry, nullptr, per);
     }
     else
         for (long long u = blockIdx.x; u < L.units; u += gridDim.x)
@@ -1902,18 +1927,19 @@ __device__ bool coop_triangle(const RSample* in, int n, const Query& o, float di
     return false;
 }
 
-// One warp: the queued output samples queue[b .. b+32) (of n) through the full
+// One warp: the queued output samples queue[b .. b+per_warp) (of n) through the full
 // path, with the warp's working lists S and shared triangle-search bits T.
 __device__ __forceinline__ void coop_group(const QParams& P, const int* __restrict__ queue, int n, int b,
                                            float4* __restrict__ qcol, int* __restrict__ ovf_queue,
-                                           int* __restrict__ ovf_count, int ovf_cap, CoopScratch& S, CoopShared& T)
+                                           int* __restrict__ ovf_count, int ovf_cap, CoopScratch& S, CoopShared& T,
+                                           int per_warp)
 {
     const int lane = threadIdx.x & 31;
     {
         // 1. per-lane traversal and leaf sort: at 2R for output samples the light
         // pass found to need it, at 1R for those that outgrew the light pass's
         // capacities (they start over from the 1R fetch)
-        const int entry = (b + lane < n) ? queue[b + lane] : -1;
+        const int entry = (lane < per_warp && b + lane < n) ? queue[b + lane] : -1;
         bool restart = entry >= 0 && (entry & kQueueRestart);
         const bool valid = entry >= 0;
         const int myq = valid ? (entry & ~kQueueRestart) : 0;
@@ -2116,8 +2142,10 @@ k_query_coop(QParams P, const int* __restrict__ queue, const int* __restrict__ q
     const int warp = blockIdx.x * kCWarps + (threadIdx.x >> 5);
     const int nwarps = gridDim.x * kCWarps;
     const int n = *queue_count;
-    for (int b = warp * 32; b < n; b += nwarps * 32)
-        coop_group(P, queue, n, b, qcol, ovf_queue, ovf_count, ovf_cap, scratch[warp], sh_tri[threadIdx.x >> 5]);
+    const int per = entries_per_warp(n, nwarps);
+    for (long long b = (long long)warp * per; b < n; b += (long long)nwarps * per)
+        coop_group(P, queue, n, (int)b, qcol, ovf_queue, ovf_count, ovf_cap, scratch[warp], sh_tri[threadIdx.x >> 5],
+                   per);
 }
 
 // Statistics pass: every output sample through the full path with the
@@ -3051,11 +3079,17 @@ static LightMap light_map(const Ctx& c, long long nq_probe = 0, int shape = kDef
 {
     LightMap L{};
     const int tw = kTileShapes[shape][0], th = kTileShapes[shape][1], sw = 32 / (tw * th);
-    if (nq_probe > 0 || c.out_spp % (4 * sw) != 0)
+    if (nq_probe > 0)
     {
-        const long long nq = nq_probe > 0 ? nq_probe : (long long)c.W * c.H * c.out_spp;
         L.mode = kMapLinear;
-        L.units = (nq + kBlock - 1) / kBlock;
+        L.units = (nq_probe + kBlock - 1) / kBlock;
+        return L;
+    }
+    if (c.out_spp % (4 * sw) != 0)
+    {
+        L.mode = kMapSingle;
+        L.tiles_x = (c.W + 7) / 8;
+        L.units = ((long long)L.tiles_x * ((c.H + 3) / 4) * c.out_spp + 3) / 4;
         return L;
     }
     L.mode = kMapTiles;
@@ -3138,8 +3172,8 @@ __device__ __forceinline__ int frame_of(const long long* __restrict__ begin, int
 // Light pass over every frame of a chunk: a block takes one unit at a time.
 // FIRST: every output sample of every frame (LightMap units), those that
 // outgrow the first tier's capacities appended to the frame's retry list (its
-// overflow queue, counters[3]); otherwise the retry lists (units of kBlock
-// entries, offsets from k_batch_retry_units), overflow to the full path.
+// overflow queue, counters[3]); otherwise the retry lists (units and entries per
+// warp from k_batch_items), overflow to the full path.
 template <bool FIRST>
 __global__ void __launch_bounds__(kBlock, FIRST ? kL1BlocksPerSM : kL2BlocksPerSM)
 k_batch_light(const FrameDesc* __restrict__ fd, const long long* __restrict__ unit_begin, int nframes,
@@ -3152,6 +3186,7 @@ k_batch_light(const FrameDesc* __restrict__ fd, const long long* __restrict__ un
     __shared__ long long sU;
     __shared__ int sF;
     const long long total = unit_begin[nframes];
+    const int per = FIRST ? 32 : (int)unit_begin[nframes + 1];
     int cur = -1;
     for (;;)
     {
@@ -3178,37 +3213,45 @@ k_batch_light(const FrameDesc* __restrict__ fd, const long long* __restrict__ un
                                                               D.counters + 2, sh, D.ovf, D.counters + 3);
         else
             light_unit<false, kL2Leaf, kL2Stack, kLightRetry>(sP, sL, u - unit_begin[f], D.counters[3], D.qcol,
-                                                              D.heavy, D.counters + 2, sh, D.ovf);
+                                                              D.heavy, D.counters + 2, sh, D.ovf, nullptr, per);
         __syncthreads();
     }
 }
 
-// Units of the retry pass: kBlock retried output samples each.
-__global__ void k_batch_retry_units(const FrameDesc* __restrict__ fd, int nframes, long long* __restrict__ unit_begin)
+// Work items of a pass over the frames' queues (counters[which]; 3: the retry
+// lists, 2: the full path): per_warp entries per warp, which is stored behind
+// the items' frame offsets.  warps_per_item: 4 for the retry pass's blocks.
+__global__ void __launch_bounds__(32)
+k_batch_items(const FrameDesc* __restrict__ fd, int nframes, int which, int warps_per_item, int nwarps,
+              long long* __restrict__ item_begin)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0)
-        return;
-    long long acc = 0;
-    for (int f = 0; f < nframes; f++)
+    const int lane = threadIdx.x;
+    long long n = 0;
+    for (int f = lane; f < nframes; f += 32)
+        n += fd[f].counters[which];
+    for (int o = 16; o > 0; o >>= 1)
+        n += __shfl_xor_sync(0xffffffffu, n, o);
+    const int per = entries_per_warp(n, nwarps), item = per * warps_per_item;
+    long long carry = 0;
+    for (int b = 0; b < nframes; b += 32)
     {
-        unit_begin[f] = acc;
-        acc += (fd[f].counters[3] + kBlock - 1) / kBlock;
+        const int f = b + lane;
+        const long long v = f < nframes ? (fd[f].counters[which] + item - 1) / item : 0;
+        long long sum = v;
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const long long x = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += x;
+        }
+        if (f < nframes)
+            item_begin[f] = carry + sum - v;
+        carry += __shfl_sync(0xffffffffu, sum, 31);
     }
-    unit_begin[nframes] = acc;
-}
-
-// Work items of the full-path pass: 32 queued output samples each.
-__global__ void k_batch_items(const FrameDesc* __restrict__ fd, int nframes, long long* __restrict__ item_begin)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0)
-        return;
-    long long acc = 0;
-    for (int f = 0; f < nframes; f++)
+    if (lane == 0)
     {
-        item_begin[f] = acc;
-        acc += (fd[f].counters[2] + 31) / 32;
+        item_begin[nframes] = carry;
+        item_begin[nframes + 1] = per;
     }
-    item_begin[nframes] = acc;
 }
 
 // Full-path pass over every frame of a chunk: a warp takes one item at a time.
@@ -3220,6 +3263,7 @@ k_batch_coop(const FrameDesc* __restrict__ fd, const long long* __restrict__ ite
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * kCWarps + (threadIdx.x >> 5);
     const long long total = item_begin[nframes];
+    const int per = (int)item_begin[nframes + 1];
     for (;;)
     {
         long long it = 0;
@@ -3230,8 +3274,8 @@ k_batch_coop(const FrameDesc* __restrict__ fd, const long long* __restrict__ ite
             break;
         const int f = frame_of(item_begin, nframes, it);
         const FrameDesc& D = fd[f];
-        coop_group(D.P, D.heavy, D.counters[2], (int)(it - item_begin[f]) * 32, D.qcol, D.ovf, D.counters + 0,
-                   (int)D.nq, scratch[warp], sh_tri[threadIdx.x >> 5]);
+        coop_group(D.P, D.heavy, D.counters[2], (int)(it - item_begin[f]) * per, D.qcol, D.ovf, D.counters + 0,
+                   (int)D.nq, scratch[warp], sh_tri[threadIdx.x >> 5], per);
     }
 }
 
@@ -3266,9 +3310,9 @@ struct BatchChunk
     int first = 0, count = 0;           // frames [first, first + count)
     FrameDesc* d_desc = nullptr;        // into BatchPlan::d_desc
     long long* d_unit_begin = nullptr;  // count + 1
-    long long* d_item_begin = nullptr;  // count + 1
+    long long* d_item_begin = nullptr;  // count + 2 (k_batch_items)
     long long* d_pix_begin = nullptr;   // count + 1
-    long long* d_retry_begin = nullptr; // count + 1
+    long long* d_retry_begin = nullptr; // count + 2
     unsigned long long* d_work = nullptr;   // [0] next light unit, [1] next full-path item, [2] next retry unit
 };
 
@@ -3481,10 +3525,10 @@ tlfr_status batch_build(BatchPlan& bp, const std::vector<BatchEntry>& entries, c
     }
     // device tables
     CKB(cudaMalloc(&bp.d_desc, sizeof(FrameDesc) * n));
-    CKB(cudaMalloc(&bp.d_offsets, sizeof(long long) * 4 * (n + bp.chunks.size())));
+    CKB(cudaMalloc(&bp.d_offsets, sizeof(long long) * (4 * n + 6 * bp.chunks.size())));
     CKB(cudaMalloc(&bp.d_work, sizeof(unsigned long long) * 3 * bp.chunks.size()));
     std::vector<long long> offs;
-    offs.reserve(4 * (n + bp.chunks.size()));
+    offs.reserve(4 * n + 6 * bp.chunks.size());
     for (size_t k = 0; k < bp.chunks.size(); k++)
     {
         BatchChunk& ch = bp.chunks[k];
@@ -3504,11 +3548,11 @@ tlfr_status batch_build(BatchPlan& bp, const std::vector<BatchEntry>& entries, c
         pb.push_back(pxl);
         offs.insert(offs.end(), ub.begin(), ub.end());
         offs.insert(offs.end(), pb.begin(), pb.end());
-        offs.insert(offs.end(), 2 * (ch.count + 1), 0LL);    // item and retry offsets, filled on the device
+        offs.insert(offs.end(), 2 * (ch.count + 2), 0LL);    // item and retry offsets, filled on the device
         ch.d_unit_begin = bp.d_offsets + base;
         ch.d_pix_begin = bp.d_offsets + base + ch.count + 1;
         ch.d_item_begin = bp.d_offsets + base + 2 * (ch.count + 1);
-        ch.d_retry_begin = bp.d_offsets + base + 3 * (ch.count + 1);
+        ch.d_retry_begin = ch.d_item_begin + ch.count + 2;
     }
     CKB(cudaMemcpy(bp.d_offsets, offs.data(), sizeof(long long) * offs.size(), cudaMemcpyHostToDevice));
     CKB(cudaMemcpy(bp.d_desc, bp.desc.data(), sizeof(FrameDesc) * n, cudaMemcpyHostToDevice));
@@ -3549,10 +3593,12 @@ tlfr_status batch_enqueue(BatchPlan& bp, cudaStream_t s, std::string& err, long 
         // queues, which the full-path pass fills only after they are read)
         k_batch_light<true><<<bp.num_sms * kL1BlocksPerSM, kBlock, 0, s>>>(ch.d_desc, ch.d_unit_begin, ch.count,
                                                                          ch.d_work + 0);
-        k_batch_retry_units<<<1, 32, 0, s>>>(ch.d_desc, ch.count, ch.d_retry_begin);
+        k_batch_items<<<1, 32, 0, s>>>(ch.d_desc, ch.count, 3, kBlock / 32, bp.num_sms * kL2BlocksPerSM * (kBlock / 32),
+                                       ch.d_retry_begin);
         k_batch_light<false><<<bp.num_sms * kL2BlocksPerSM, kBlock, 0, s>>>(ch.d_desc, ch.d_retry_begin, ch.count,
                                                                           ch.d_work + 2);
-        k_batch_items<<<1, 32, 0, s>>>(ch.d_desc, ch.count, ch.d_item_begin);
+        k_batch_items<<<1, 32, 0, s>>>(ch.d_desc, ch.count, 2, 1, bp.num_sms * kCoopBlocksPerSM * kCWarps,
+                                       ch.d_item_begin);
         k_batch_coop<<<bp.num_sms * kCoopBlocksPerSM, kCWarps * 32, 0, s>>>(ch.d_desc, ch.d_item_begin, ch.count,
                                                                            ch.d_work + 1,
                                                                            reinterpret_cast<CoopScratch*>(bp.coop_scratch));
