@@ -186,12 +186,19 @@ constexpr int kOffMean = kNumTrain;               // input standardisation (fixe
 constexpr int kOffInvStd = kOffMean + kF;
 constexpr int kNumParams = kOffInvStd + kF;
 
-// BF16 operand block: w1 [64][16], w2 [64][64], w2 transposed [64][64], w3 padded to [8][64]
-constexpr int kHW1 = 0;
-constexpr int kHW2 = kHW1 + kH * kK1;
-constexpr int kHW2T = kHW2 + kH * kH;
-constexpr int kHW3 = kHW2T + kH * kH;
-constexpr int kNumHalf = kHW3 + 8 * kH;
+// BF16 operand block: the B operands (16 x 8) of every mma, fragment by fragment
+// as the lanes hold them: lane (g, t) of fragment f has elements (k, n) = (2t, g),
+// (2t + 1, g), (2t + 8, g), (2t + 9, g) in 8 bytes at (f * 32 + lane).  A fragment
+// is then one coalesced 64-bit load, two L1 wavefronts; read from the row-major
+// matrices it took two loads of eight each, which bound inference (2.07 M rows:
+// 329 us, now 135).
+// Fragments: layer 1 by output tile; layer 2 by (output tile, k tile), W2 and then
+// its transpose; layer 3, padded to 8 outputs, by k tile.
+constexpr int kFragW1 = 0;
+constexpr int kFragW2 = kFragW1 + 8;
+constexpr int kFragW2T = kFragW2 + 32;
+constexpr int kFragW3 = kFragW2T + 32;
+constexpr int kNumHalf = (kFragW3 + 4) * 128;
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
@@ -211,14 +218,12 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// B operand (16 x 8, "col": element (k, n) at n * ld + k) from a row-major
-// [n][k] BF16 matrix: rows n0 + g, columns k0 + 2t (+1) and k0 + 2t + 8 (+1).
-__device__ __forceinline__ void load_b(const __nv_bfloat16* w, int ld, int n0, int k0, int g, int t, uint32_t& b0,
-                                       uint32_t& b1)
+// This lane's part of B fragment f.
+__device__ __forceinline__ void load_b(const __nv_bfloat16* w, int f, uint32_t& b0, uint32_t& b1)
 {
-    const __nv_bfloat16* r = w + (size_t)(n0 + g) * ld + k0 + 2 * t;
-    b0 = *reinterpret_cast<const uint32_t*>(r);
-    b1 = *reinterpret_cast<const uint32_t*>(r + 8);
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(w) + f * 32 + (threadIdx.x & 31));
+    b0 = v.x;
+    b1 = v.y;
 }
 
 // Accumulator tiles c[2kk], c[2kk+1] (16 x 8 each) as the A operand of k-tile kk.
@@ -231,7 +236,7 @@ __device__ __forceinline__ void acc_to_a(const float (&c0)[4], const float (&c1)
 }
 
 // Forward pass of one 16-row tile.  Lane (g = lane/4, t = lane%4) holds rows
-// g and g + 8.  Outputs: h1, h2 after ReLU, rounded to BF16 (the values the
+// g and g + 8, whose features are at row[0] and row[1] (zero where not valid).  Outputs: h1, h2 after ReLU, rounded to BF16 (the values the
 // next layer multiplies), columns 8j + 2t (+1); logits y for rows g and g+8
 // (valid on lanes with t == 0).
 struct Tile
@@ -242,60 +247,69 @@ struct Tile
 };
 
 __device__ __forceinline__ void tile_forward(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Wh,
-                                             const float* __restrict__ feats, const int* rows, int nrows, Tile& T)
+                                             const float* __restrict__ feats, const int (&row)[2], const bool (&valid)[2],
+                                             Tile& T)
 {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int t = threadIdx.x & 3;
     float xv[2][2];
+#pragma unroll
     for (int h = 0; h < 2; h++)
     {
-        const int r = g + 8 * h;
-        for (int q = 0; q < 2; q++)
-        {
-            const int col = 2 * t + q;
-            float v = 0.0f;
-            if (r < nrows)
-                v = (feats[(size_t)rows[r] * kF + col] - P[kOffMean + col]) * P[kOffInvStd + col];
-            xv[h][q] = v;
-        }
+        float2 f = make_float2(0, 0);
+        if (valid[h])
+            f = *reinterpret_cast<const float2*>(feats + (size_t)row[h] * kF + 2 * t);
+        const int col = 2 * t;
+        xv[h][0] = valid[h] ? (f.x - P[kOffMean + col]) * P[kOffInvStd + col] : 0.0f;
+        xv[h][1] = valid[h] ? (f.y - P[kOffMean + col + 1]) * P[kOffInvStd + col + 1] : 0.0f;
     }
     T.x[0] = pack_bf16(xv[0][0], xv[0][1]);
     T.x[1] = pack_bf16(xv[1][0], xv[1][1]);
     T.x[2] = 0;
     T.x[3] = 0;
     // layer 1
+#pragma unroll
     for (int j = 0; j < 8; j++)
     {
         float c[4] = { 0, 0, 0, 0 };
         uint32_t b0, b1;
-        load_b(Wh + kHW1, kK1, 8 * j, 0, g, t, b0, b1);
+        load_b(Wh, kFragW1 + j, b0, b1);
         mma16816(c, T.x, b0, b1);
+        const float2 bias = *reinterpret_cast<const float2*>(P + kOffB1 + 8 * j + 2 * t);
+#pragma unroll
         for (int q = 0; q < 4; q++)
-            T.h1[j][q] = bf16_round(fmaxf(c[q] + P[kOffB1 + 8 * j + 2 * t + (q & 1)], 0.0f));
+            T.h1[j][q] = bf16_round(fmaxf(c[q] + (q & 1 ? bias.y : bias.x), 0.0f));
     }
     // layer 2
     uint32_t a[4][4];
+#pragma unroll
     for (int kk = 0; kk < 4; kk++)
         acc_to_a(T.h1[2 * kk], T.h1[2 * kk + 1], a[kk]);
+#pragma unroll
     for (int j = 0; j < 8; j++)
     {
         float c[4] = { 0, 0, 0, 0 };
-        for (int kk = 0; kk < 4; kk++)
+#pragma unroll
+    for (int kk = 0; kk < 4; kk++)
         {
             uint32_t b0, b1;
-            load_b(Wh + kHW2, kH, 8 * j, 16 * kk, g, t, b0, b1);
+            load_b(Wh, kFragW2 + 4 * j + kk, b0, b1);
             mma16816(c, a[kk], b0, b1);
         }
+        const float2 bias = *reinterpret_cast<const float2*>(P + kOffB2 + 8 * j + 2 * t);
+#pragma unroll
         for (int q = 0; q < 4; q++)
-            T.h2[j][q] = bf16_round(fmaxf(c[q] + P[kOffB2 + 8 * j + 2 * t + (q & 1)], 0.0f));
+            T.h2[j][q] = bf16_round(fmaxf(c[q] + (q & 1 ? bias.y : bias.x), 0.0f));
     }
     // layer 3 (one output column of an 8-wide tile)
+#pragma unroll
     for (int kk = 0; kk < 4; kk++)
         acc_to_a(T.h2[2 * kk], T.h2[2 * kk + 1], a[kk]);
     float c[4] = { 0, 0, 0, 0 };
+#pragma unroll
     for (int kk = 0; kk < 4; kk++)
     {
         uint32_t b0, b1;
-        load_b(Wh + kHW3, kH, 0, 16 * kk, g, t, b0, b1);
+        load_b(Wh, kFragW3 + kk, b0, b1);
         mma16816(c, a[kk], b0, b1);
     }
     T.y0 = c[0] + P[kOffB3];
@@ -310,15 +324,14 @@ __global__ void __launch_bounds__(128) k_mlp_infer(const float* __restrict__ P, 
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    int rows[16];
     for (long long tile = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile * 16 < n; tile += warps)
     {
         const long long r0 = tile * 16;
         const int nrows = (int)min(16LL, n - r0);
-        for (int r = 0; r < 16; r++)
-            rows[r] = (int)(r0 + (r < nrows ? r : 0));
+        const int row[2] = { (int)(r0 + g), (int)(r0 + g + 8) };
+        const bool valid[2] = { g < nrows, g + 8 < nrows };
         Tile T;
-        tile_forward(P, Wh, feats, rows, nrows, T);
+        tile_forward(P, Wh, feats, row, valid, T);
         if (t == 0)
         {
             if (g < nrows)
@@ -352,16 +365,23 @@ constexpr int kTrainWarps = 4;
 // minibatch; gradients are added into grad (FP32, kNumTrain).  Rows are the
 // minibatch rows: row k = batch_row(seed, step, k, n), or k itself when
 // all_rows is set (the gradient over exactly rows 0..batch-1).
+// A block takes kTrainWarps tiles of 16 rows at a time: each warp runs one tile
+// forward and back and stages what the weight gradients contract over the rows;
+// then warp w accumulates rows 16w..16w+15 of dL/dW2 and dL/dW1 over all the
+// block's tiles in its mma accumulators, kept for the whole launch.  (Adding every
+// tile's products to shared memory with float atomics took 544 us for 262144
+// rows; this 169 us, 121 with the weights read as fragments.)
 __global__ void __launch_bounds__(kTrainWarps * 32)
 k_mlp_train(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Wh, const float* __restrict__ feats,
             const float* __restrict__ labels, int n, int batch, unsigned seed, unsigned step, int all_rows,
             float* __restrict__ grad, float* __restrict__ loss_out)
 {
+    static_assert(kTrainWarps * 16 == kH, "a warp owns 16 rows of the weight gradients");
     __shared__ float s_grad[kNumTrain];
     __shared__ __nv_bfloat16 s_h1[kTrainWarps][16][kH];
     __shared__ __nv_bfloat16 s_dh2[kTrainWarps][16][kH];
     __shared__ __nv_bfloat16 s_dh1[kTrainWarps][16][kH];
-    __shared__ __nv_bfloat16 s_x[kTrainWarps][16][kK1];
+    __shared__ __nv_bfloat16 s_x[kTrainWarps][16][kF];
     __shared__ float s_loss;
     for (int i = threadIdx.x; i < kNumTrain; i += blockDim.x)
         s_grad[i] = 0.0f;
@@ -371,153 +391,153 @@ k_mlp_train(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Wh, c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const float inv_batch = 1.0f / (float)batch;
     float loss = 0.0f;
-    int rows[16];
-    for (int tile = blockIdx.x * kTrainWarps + warp; tile * 16 < batch; tile += gridDim.x * kTrainWarps)
+    float c2[8][4] = {}, c1[4] = {};        // this warp's rows of dL/dW2 and dL/dW1
+    float gw3[8][2] = {}, gb2[8][2] = {}, gb1[8][2] = {}, gb3 = 0.0f;     // this lane's rows' sums
+    for (long long first = (long long)blockIdx.x * kTrainWarps * 16; first < batch;
+         first += (long long)gridDim.x * kTrainWarps * 16)
     {
-        const int k0 = tile * 16;
-        const int nrows = min(16, batch - k0);
-        for (int r = 0; r < 16; r++)
+        const long long k0 = first + warp * 16;
+        const int nrows = (int)max(0LL, min(16LL, batch - k0));
+        const bool valid[2] = { g < nrows, g + 8 < nrows };
+        int row[2];
+        for (int h = 0; h < 2; h++)
         {
-            const int k = k0 + (r < nrows ? r : 0);
-            rows[r] = all_rows ? k : batch_row(seed, step, (unsigned)k, (unsigned)n);
+            const int k = valid[h] ? (int)(k0 + g + 8 * h) : 0;
+            row[h] = all_rows ? k : batch_row(seed, step, (unsigned)k, (unsigned)n);
         }
         Tile T;
-        tile_forward(P, Wh, feats, rows, nrows, T);
+        tile_forward(P, Wh, feats, row, valid, T);
         // dL/dy = (p - label) / batch for rows g and g + 8, broadcast to the lane group
         float dy0 = 0.0f, dy8 = 0.0f;
         if (t == 0)
         {
-            if (g < nrows)
+            if (valid[0])
             {
-                const float p = sigmoid(T.y0), lab = labels[rows[g]];
+                const float p = sigmoid(T.y0), lab = labels[row[0]];
                 dy0 = (p - lab) * inv_batch;
                 loss -= (lab * logf(fmaxf(p, 1e-7f)) + (1 - lab) * logf(fmaxf(1 - p, 1e-7f))) * inv_batch;
             }
-            if (g + 8 < nrows)
+            if (valid[1])
             {
-                const float p = sigmoid(T.y8), lab = labels[rows[g + 8]];
+                const float p = sigmoid(T.y8), lab = labels[row[1]];
                 dy8 = (p - lab) * inv_batch;
                 loss -= (lab * logf(fmaxf(p, 1e-7f)) + (1 - lab) * logf(fmaxf(1 - p, 1e-7f))) * inv_batch;
             }
+            gb3 += dy0 + dy8;
         }
         dy0 = __shfl_sync(0xffffffffu, dy0, lane & ~3);
         dy8 = __shfl_sync(0xffffffffu, dy8, lane & ~3);
         // layer 3: grad w3, b3; dh2 = dy * w3 * relu'(h2)
         float dh2[8][4];
+#pragma unroll
         for (int j = 0; j < 8; j++)
+#pragma unroll
             for (int q = 0; q < 2; q++)
             {
                 const int col = 8 * j + 2 * t + q;
                 const float w3 = bf16_round(P[kOffW3 + col]);
-                const float gw = sum_groups(dy0 * T.h2[j][q] + dy8 * T.h2[j][q + 2]);
-                if (g == 0)
-                    atomicAdd(&s_grad[kOffW3 + col], gw);
+                gw3[j][q] += dy0 * T.h2[j][q] + dy8 * T.h2[j][q + 2];
                 dh2[j][q] = T.h2[j][q] > 0.0f ? bf16_round(dy0 * w3) : 0.0f;
                 dh2[j][q + 2] = T.h2[j][q + 2] > 0.0f ? bf16_round(dy8 * w3) : 0.0f;
-                const float gb = sum_groups(dh2[j][q] + dh2[j][q + 2]);
-                if (g == 0)
-                    atomicAdd(&s_grad[kOffB2 + col], gb);
+                gb2[j][q] += dh2[j][q] + dh2[j][q + 2];
             }
-        {
-            const float gb3 = sum_groups(t == 0 ? dy0 + dy8 : 0.0f);
-            if (lane == 0)
-                atomicAdd(&s_grad[kOffB3], gb3);
-        }
         // dh1 = dh2 * W2 (row-major [n][k]; the B operand is W2 transposed) * relu'(h1)
         uint32_t a[4][4];
+#pragma unroll
         for (int kk = 0; kk < 4; kk++)
             acc_to_a(dh2[2 * kk], dh2[2 * kk + 1], a[kk]);
-        float dh1[8][4];
+        __syncthreads();        // the previous group's staged tiles have been read
+#pragma unroll
         for (int j = 0; j < 8; j++)
         {
             float c[4] = { 0, 0, 0, 0 };
+#pragma unroll
             for (int kk = 0; kk < 4; kk++)
             {
                 uint32_t b0, b1;
-                load_b(Wh + kHW2T, kH, 8 * j, 16 * kk, g, t, b0, b1);
+                load_b(Wh, kFragW2T + 4 * j + kk, b0, b1);
                 mma16816(c, a[kk], b0, b1);
             }
+            float dh1[4];
+#pragma unroll
             for (int q = 0; q < 4; q++)
-                dh1[j][q] = T.h1[j][q] > 0.0f ? bf16_round(c[q]) : 0.0f;
+                dh1[q] = T.h1[j][q] > 0.0f ? bf16_round(c[q]) : 0.0f;
+#pragma unroll
             for (int q = 0; q < 2; q++)
+                gb1[j][q] += dh1[q] + dh1[q + 2];
+            // stage h1, dh2, dh1 (row-major [row][col]) for the weight gradients,
+            // which contract over the rows
+#pragma unroll
+            for (int h = 0; h < 2; h++)
             {
-                const float gb = sum_groups(dh1[j][q] + dh1[j][q + 2]);
-                if (g == 0)
-                    atomicAdd(&s_grad[kOffB1 + 8 * j + 2 * t + q], gb);
+                const int r = g + 8 * h, col = 8 * j + 2 * t;
+                *reinterpret_cast<uint32_t*>(&s_h1[warp][r][col]) = pack_bf16(T.h1[j][2 * h], T.h1[j][2 * h + 1]);
+                *reinterpret_cast<uint32_t*>(&s_dh2[warp][r][col]) = pack_bf16(dh2[j][2 * h], dh2[j][2 * h + 1]);
+                *reinterpret_cast<uint32_t*>(&s_dh1[warp][r][col]) = pack_bf16(dh1[2 * h], dh1[2 * h + 1]);
             }
         }
-        // stage h1, dh2, dh1, x (row-major [row][col]) for the weight gradients,
-        // which contract over the rows
-        for (int j = 0; j < 8; j++)
-            for (int q = 0; q < 4; q++)
-            {
-                const int r = g + 8 * (q >> 1), col = 8 * j + 2 * t + (q & 1);
-                s_h1[warp][r][col] = __float2bfloat16_rn(T.h1[j][q]);
-                s_dh2[warp][r][col] = __float2bfloat16_rn(dh2[j][q]);
-                s_dh1[warp][r][col] = __float2bfloat16_rn(dh1[j][q]);
-            }
-        {
-            const __nv_bfloat162* xs = reinterpret_cast<const __nv_bfloat162*>(T.x);
-            for (int q = 0; q < 2; q++)
-            {
-                s_x[warp][g + 8 * q][2 * t] = xs[q].x;
-                s_x[warp][g + 8 * q][2 * t + 1] = xs[q].y;
-                s_x[warp][g + 8 * q][2 * t + 8] = __float2bfloat16_rn(0.0f);
-                s_x[warp][g + 8 * q][2 * t + 9] = __float2bfloat16_rn(0.0f);
-            }
-        }
-        __syncwarp();
+        *reinterpret_cast<uint32_t*>(&s_x[warp][g][2 * t]) = T.x[0];
+        *reinterpret_cast<uint32_t*>(&s_x[warp][g + 8][2 * t]) = T.x[1];
+        __syncthreads();
         // grad W2[n][k] = sum_rows dh2[row][n] * h1[row][k]; grad W1[n][k] = sum_rows dh1[row][n] * x[row][k].
         // A = (dh)^T tile [n][row] (16 x 16), B = (h1 or x) as (k = row, n = col).
-        auto at = [&](__nv_bfloat16 (*m)[kH], int r, int c) {
-            uint32_t lo = reinterpret_cast<const uint16_t&>(m[r][c]);
-            return lo;
+        auto at = [&](const __nv_bfloat16* m, int ld, int r, int c) {
+            return (uint32_t)reinterpret_cast<const uint16_t&>(m[r * ld + c]) |
+                   ((uint32_t)reinterpret_cast<const uint16_t&>(m[(r + 1) * ld + c]) << 16);
         };
-        for (int mt = 0; mt < 4; mt++)
+        for (int rt = 0; rt < kTrainWarps; rt++)
         {
             uint32_t A2[4], A1[4];
+#pragma unroll
             for (int q = 0; q < 4; q++)
             {
-                const int nn = 16 * mt + g + 8 * (q & 1);
+                const int nn = 16 * warp + g + 8 * (q & 1);
                 const int rr = 2 * t + 8 * (q >> 1);
-                A2[q] = at(s_dh2[warp], rr, nn) | (at(s_dh2[warp], rr + 1, nn) << 16);
-                A1[q] = at(s_dh1[warp], rr, nn) | (at(s_dh1[warp], rr + 1, nn) << 16);
+                A2[q] = at(&s_dh2[rt][0][0], kH, rr, nn);
+                A1[q] = at(&s_dh1[rt][0][0], kH, rr, nn);
             }
+#pragma unroll
             for (int j = 0; j < 8; j++)
             {
                 const int kc = 8 * j + g;
-                const uint32_t b0 = at(s_h1[warp], 2 * t, kc) | (at(s_h1[warp], 2 * t + 1, kc) << 16);
-                const uint32_t b1 = at(s_h1[warp], 2 * t + 8, kc) | (at(s_h1[warp], 2 * t + 9, kc) << 16);
-                float c[4] = { 0, 0, 0, 0 };
-                mma16816(c, A2, b0, b1);
-                for (int q = 0; q < 4; q++)
-                {
-                    const int nn = 16 * mt + g + 8 * (q >> 1), kcol = 8 * j + 2 * t + (q & 1);
-                    atomicAdd(&s_grad[kOffW2 + nn * kH + kcol], c[q]);
-                }
+                mma16816(c2[j], A2, at(&s_h1[rt][0][0], kH, 2 * t, kc), at(&s_h1[rt][0][0], kH, 2 * t + 8, kc));
             }
+            // x columns 0..7
+            mma16816(c1, A1, at(&s_x[rt][0][0], kF, 2 * t, g), at(&s_x[rt][0][0], kF, 2 * t + 8, g));
+        }
+    }
+    // the weight gradients, each element held by one lane of the block
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+        const int nn = 16 * warp + g + 8 * (q >> 1);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            s_grad[kOffW2 + nn * kH + 8 * j + 2 * t + (q & 1)] = c2[j][q];
+        s_grad[kOffW1 + nn * kK1 + 2 * t + (q & 1)] = c1[q];
+    }
+    // the others, summed over the block's warps
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+        {
+            const float w3 = sum_groups(gw3[j][q]), b2 = sum_groups(gb2[j][q]), b1 = sum_groups(gb1[j][q]);
+            if (g == 0)
             {
-                const int kc = g;   // x columns 0..7
-                const uint32_t b0 = reinterpret_cast<const uint16_t&>(s_x[warp][2 * t][kc]) |
-                                    ((uint32_t)reinterpret_cast<const uint16_t&>(s_x[warp][2 * t + 1][kc]) << 16);
-                const uint32_t b1 = reinterpret_cast<const uint16_t&>(s_x[warp][2 * t + 8][kc]) |
-                                    ((uint32_t)reinterpret_cast<const uint16_t&>(s_x[warp][2 * t + 9][kc]) << 16);
-                float c[4] = { 0, 0, 0, 0 };
-                mma16816(c, A1, b0, b1);
-                for (int q = 0; q < 4; q++)
-                {
-                    const int nn = 16 * mt + g + 8 * (q >> 1), kcol = 2 * t + (q & 1);
-                    atomicAdd(&s_grad[kOffW1 + nn * kK1 + kcol], c[q]);
-                }
+                const int col = 8 * j + 2 * t + q;
+                atomicAdd(&s_grad[kOffW3 + col], w3);
+                atomicAdd(&s_grad[kOffB2 + col], b2);
+                atomicAdd(&s_grad[kOffB1 + col], b1);
             }
         }
-        __syncwarp();
-    }
+    gb3 = sum_groups(gb3);
     loss = sum_groups(loss);
-    loss += __shfl_xor_sync(0xffffffffu, loss, 1);
-    loss += __shfl_xor_sync(0xffffffffu, loss, 2);
     if (lane == 0)
+    {
+        atomicAdd(&s_grad[kOffB3], gb3);
         atomicAdd(&s_loss, loss);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < kNumTrain; i += blockDim.x)
         if (s_grad[i] != 0.0f)
@@ -547,21 +567,17 @@ __global__ void k_pack(const float* __restrict__ P, __nv_bfloat16* __restrict__ 
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kNumHalf; i += gridDim.x * blockDim.x)
     {
+        const int f = i >> 7, lane = (i >> 2) & 31;
+        const int n = lane >> 2, k = 2 * (lane & 3) + (i & 1) + 8 * ((i >> 1) & 1);
         float v;
-        if (i < kHW2)
-            v = P[kOffW1 + i];
-        else if (i < kHW2T)
-            v = P[kOffW2 + (i - kHW2)];
-        else if (i < kHW3)
-        {
-            const int e = i - kHW2T, r = e / kH, c = e % kH;   // W2T[r][c] = W2[c][r]
-            v = P[kOffW2 + c * kH + r];
-        }
+        if (f < kFragW2)
+            v = P[kOffW1 + (8 * f + n) * kK1 + k];
+        else if (f < kFragW2T)
+            v = P[kOffW2 + (8 * ((f - kFragW2) >> 2) + n) * kH + 16 * ((f - kFragW2) & 3) + k];
+        else if (f < kFragW3)
+            v = P[kOffW2 + (16 * ((f - kFragW2T) & 3) + k) * kH + 8 * ((f - kFragW2T) >> 2) + n];
         else
-        {
-            const int e = i - kHW3, r = e / kH, c = e % kH;
-            v = r == 0 ? P[kOffW3 + c] : 0.0f;
-        }
+            v = n == 0 ? P[kOffW3 + 16 * (f - kFragW3) + k] : 0.0f;
         Wh[i] = __float2bfloat16_rn(v);
     }
 }
