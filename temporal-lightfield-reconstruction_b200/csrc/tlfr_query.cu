@@ -65,7 +65,7 @@ struct QParams
     float c0, c1;               // refocused CoC coefficients
     float disp0;
     int   lens_filter, time_filter;
-    float r2_wide, min_w;       // may_accept()'s bounds at 1R (accept_bound())
+    float r2_wide, r2_wide2, min_w;     // may_accept()'s bounds at 1R and 2R (accept_bound())
     float one;                  // 1 (eval2())
     const unsigned char* route_fast;   // per pixel, nonzero: first-surface fast path (or null)
 };
@@ -781,9 +781,8 @@ __device__ __forceinline__ void fw_insertion_sort(LaneLeaves& a, int start, int 
 // output sample and no stack.
 // All lanes take each step together; the keys are read after the traversal, as
 // neighbouring lanes reach their leaves at different steps.
-template <bool PROBE, int LEAF, int STACK>
-__device__ __forceinline__ int light_collect(const QParams& P, const Query& o, float R, bool valid,
-                                             LightShared<LEAF, STACK>& S)
+template <bool PROBE, int LEAF, int STACK, class SHARED>
+__device__ __forceinline__ int light_collect(const QParams& P, const Query& o, float R, bool valid, SHARED& S)
 {
     static_assert(LEAF <= 32, "the warp's scan holds one leaf per lane");
     constexpr int kNone = (int)0x80000000;
@@ -1642,10 +1641,13 @@ constexpr int kTriWords = (kTriMax + 31) / 32;
 
 // Per-warp shared memory of the full path: the coverage search's bit rows, and
 // the sameSurface values of the current group of 32 leaves ([value][leaf]).
-struct CoopShared
+struct TriShared
 {
     unsigned row[kTriWords];                    // samples l > m within 2*dispersion of m
     unsigned mask[5 * kTriWords];               // quadrant patterns 3, 6, 9, 12; within dispersion
+};
+struct CoopShared : TriShared
+{
     float sv[16][32];
 };
 
@@ -1834,11 +1836,12 @@ __device__ __forceinline__ void coop_reverse(RSample* a, int lo, int hi)     // 
 // length before the edge functions.
 
 
-__device__ bool coop_triangle(const RSample* in, int n, const Query& o, float dispersion, CoopShared& T)
+__device__ bool coop_triangle(const RSample* in, int n, const Query& o, float dispersion, TriShared& T)
 {
     const int lane = threadIdx.x & 31;
     const int W = (n + 31) >> 5;
     const float side = 2 * dispersion;
+    unsigned any3 = 0, any6 = 0, any9 = 0, any12 = 0;
     for (int w = 0; w < W; w++)
     {
         const int i = (w << 5) + lane;
@@ -1852,6 +1855,7 @@ __device__ bool coop_triangle(const RSample* in, int n, const Query& o, float di
         const unsigned q9 = __ballot_sync(0xffffffffu, v && r.rpos == 9);
         const unsigned q12 = __ballot_sync(0xffffffffu, v && r.rpos == 12);
         const unsigned nr = __ballot_sync(0xffffffffu, near);
+        any3 |= q3; any6 |= q6; any9 |= q9; any12 |= q12;
         if (lane == 0)
         {
             T.mask[0 * kTriWords + w] = q3; T.mask[1 * kTriWords + w] = q6;
@@ -1859,6 +1863,10 @@ __device__ bool coop_triangle(const RSample* in, int n, const Query& o, float di
             T.mask[4 * kTriWords + w] = nr;
         }
     }
+    // all four quadrant bits take samples in opposite quadrants: 143 -> 125 ms for
+    // the full path at 960x540x8, 40.7 -> 32.8 ms at 962x543x4
+    if (!((any3 && any12) || (any6 && any9)))
+        return false;
     for (int m = 0; m < n - 2; m++)
     {
         const RSample r0 = in[m];
@@ -1925,6 +1933,354 @@ __device__ bool coop_triangle(const RSample* in, int n, const Query& o, float di
         __syncwarp();       // the next row overwrites T.row
     }
     return false;
+}
+
+// The rest of one output sample by the warp, from its surfaces' accepted samples
+// on: tiny-surface merging, the surfaces front to back, and the colour.
+__device__ __forceinline__ void coop_resolve(const QParams& P, const Query& o, float dispersion, bool fetch2R,
+                                             RSample* rs, Surf* surf, int nsurf, TriShared& T,
+                                             float4* __restrict__ qcol, int qj)
+{
+    const int lane = threadIdx.x & 31;
+    // tiny-surface merging (RO.cpp:137-156): dst.samples += src.samples
+    for (int sidx = 0; fetch2R && sidx < nsurf - 1; sidx++)
+    {
+        Surf src = surf[sidx], dst = surf[sidx + 1];
+        __syncwarp();
+        if (src.n < 4)
+        {
+            const int lo = src.start, mid = src.start + src.n, hi = dst.start + dst.n;
+            if (src.n > 0 && mid == dst.start)
+            {
+                coop_reverse(rs, lo, mid);
+                coop_reverse(rs, mid, hi);
+                coop_reverse(rs, lo, hi);
+            }
+            if (lane == 0)
+            {
+                Surf& d = surf[sidx + 1];
+                d.start = lo;
+                d.n = hi - lo;
+                if (src.minDist < dst.minDist)
+                {
+                    d.minDist = src.minDist;
+                    d.minIndex = src.minIndex;
+                }
+                surf[sidx].n = 0;
+            }
+            __syncwarp();
+        }
+    }
+    // resolve (RO.cpp:165-304)
+    bool found = false;
+    float4 res = make_float4(0, 0, 0, 0);
+    float nearestDist = kF32Max;
+    int nearS = -1, nearI = 1;
+    for (int sidx = 0; sidx < nsurf && !found; sidx++)
+    {
+        const Surf sf = surf[sidx];
+        const int cnt = sf.n;
+        if (cnt == 0)
+            continue;
+        const RSample* in = rs + sf.start;
+        if (sf.minDist < nearestDist)
+        {
+            nearestDist = sf.minDist;
+            nearS = sidx; nearI = sf.minIndex;
+        }
+        if (!fetch2R || sf.minDist < 0.f || sidx == nsurf - 1)
+            found = true;
+        if (cnt >= kTriMax)
+            found = true;
+        if (!found && cnt >= 3)
+            found = coop_triangle(in, cnt, o, dispersion, T);
+        if (found)
+        {
+            // tent filter (RO.cpp:274-294): products in parallel, summed
+            // in sample order by every lane from shuffles
+            res = make_float4(0, 0, 0, 0);
+            for (int kb = 0; kb < cnt; kb += 32)
+            {
+                const int k = kb + lane;
+                float4 pr = make_float4(0, 0, 0, 0);
+                bool inc = false;
+                if (k < cnt)
+                {
+                    const RSample r = in[k];
+                    const float dx = o.x - r.x, dy = o.y - r.y;
+                    const float weight = 1 - len2(dx, dy) / dispersion;
+                    if (weight > 0)
+                    {
+                        const float4 c = P.s_col[r.index];
+                        pr = make_float4(c.x * weight, c.y * weight, c.z * weight, c.w * weight);
+                        inc = true;
+                    }
+                }
+                for (unsigned mi = __ballot_sync(0xffffffffu, inc); mi; mi &= mi - 1)
+                {
+                    const int src = __ffs(mi) - 1;
+                    res.x += __shfl_sync(0xffffffffu, pr.x, src);
+                    res.y += __shfl_sync(0xffffffffu, pr.y, src);
+                    res.z += __shfl_sync(0xffffffffu, pr.z, src);
+                    res.w += __shfl_sync(0xffffffffu, pr.w, src);
+                }
+            }
+            const float oow = rcp(res.w);
+            res.x *= oow; res.y *= oow; res.z *= oow; res.w *= oow;
+            nearS = sidx; nearI = sf.minIndex;
+        }
+    }
+    if (lane == 0)
+    {
+        float4 out = make_float4(0, 0, 0, 0);
+        if (nearS != -1)
+        {
+            if (res.w == 0)
+                res = P.s_col[rs[surf[nearS].start + nearI].index];
+            if (P.lens_filter == 1)
+            {
+                float g = gaussian(o.u, 0.5f, 0) * gaussian(o.v, 0.5f, 0);
+                res.x *= g; res.y *= g; res.z *= g; res.w *= g;
+            }
+            if (P.time_filter == 1)
+            {
+                float g = gaussian(o.t, 0.25f, 0.5f);
+                res.x *= g; res.y *= g; res.z *= g; res.w *= g;
+            }
+            out = res;
+        }
+        qcol[qj] = out;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Pass 2, first kernel: queued output samples whose 2R fetch reaches at most 32
+// leaves and kFullEntries samples that may_accept() (the rest, restarted ones and
+// those with nothing within 2R go on to k_query_coop): full path 51.6 -> 40.7 ms at
+// 962x543x4, 146.5 -> 143.4 at 960x540x8.  The light pass's traversal
+// and scan at 2R, with the lists of one output sample at a time in shared memory;
+// the accepted samples are compacted in order, and surfaces open where a leaf is
+// not one surface with a leaf since the open one began (RO.cpp:412-503).
+// ---------------------------------------------------------------------------
+constexpr int kFullLeaf = 32, kFullStack = 32, kFullEntries = 192;
+constexpr int kFullBlocksPerSM = 6;
+struct FullScan
+{
+    float         values[2][16];
+    // accepted samples; the samples to test (sample, leaf) lie in the second half and are
+    // read 32 at a time before the accepted ones of these are written
+    RSample       rs[kFullEntries];
+    unsigned char leaf_of[kFullEntries];        // accepted sample's leaf
+    Surf          surf[kFullLeaf];
+    TriShared     tri;
+};
+struct FullShared
+{
+    alignas(16) float query[32][5];
+    alignas(16) int leaf[kFullLeaf][32];
+    union
+    {
+        int   stack[kFullStack][32];
+        float key[kFullLeaf][32];
+        FullScan scan;
+    };
+};
+
+__device__ __forceinline__ void full_unit(const QParams& P, const int* __restrict__ queue, long long n, long long b,
+                                          int per_warp, float4* __restrict__ qcol, int* __restrict__ next,
+                                          int* __restrict__ next_count, FullShared& S)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u, upto = (2u << lane) - 1u;
+    FullScan& T = S.scan;
+    int2* entries = reinterpret_cast<int2*>(T.rs + kFullEntries / 2);
+    const int entry = lane < per_warp && b + lane < n ? queue[b + lane] : -1;
+    const bool valid = entry >= 0 && !(entry & kQueueRestart);
+    const int qid = valid ? entry : 0;
+    Query o{};
+    if (valid)
+        o = query_of(P, qid);
+    __syncwarp();       // the previous unit's lists have been read
+    {
+        float* qp = S.query[lane];
+        qp[0] = o.x; qp[1] = o.y; qp[2] = o.u; qp[3] = o.v; qp[4] = o.t;
+    }
+    __syncwarp();
+    const float R = P.disp0 * 2, R2 = R * R;
+    const float RANGE = 1.0f / sqrtf(128.0f);
+    const int nl = light_collect<false, kFullLeaf, kFullStack>(P, o, R, valid, S);
+    __syncwarp();
+    unsigned onward = __ballot_sync(0xffffffffu, entry >= 0 && nl <= 0);
+    for (unsigned todo = __ballot_sync(0xffffffffu, nl > 0); todo; todo &= todo - 1)
+    {
+        const int j = __ffs(todo) - 1;
+        const float* qj = S.query[j];
+        const Query oj{ qj[0], qj[1], qj[2], qj[3], qj[4] };
+        const int nlj = __shfl_sync(0xffffffffu, nl, j);
+        const int qidj = __shfl_sync(0xffffffffu, qid, j);
+        // the scan of light_unit() at 2R
+        NodePairs leaf;
+        int my_n = 0;
+        if (lane < nlj)
+        {
+            leaf = load_pairs(P.nodes, S.leaf[lane][j ^ lane]);
+            my_n = leaf.s1 - leaf.s0;
+        }
+        int my_f = my_n;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1)
+        {
+            const int v = __shfl_up_sync(0xffffffffu, my_f, off);
+            if (lane >= off)
+                my_f += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, my_f, 31);
+        my_f = lane < nlj ? my_f - my_n : 0x7fffffff;
+        const int my_d = lane < nlj ? leaf.s0 - my_f : 0;
+        int cnt = 0, kbase = -1;
+        for (int base = 0; base < total; base += 32)
+        {
+            const unsigned at = (unsigned)(my_f - base);
+            const unsigned starts = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+            const int k = kbase + __popc(starts & upto);
+            kbase += __popc(starts);
+            const int i = base + lane + __shfl_sync(0xffffffffu, my_d, k);
+            bool may = false;
+            if (base + lane < total)
+            {
+                float4 pos, mot;
+                load_sample(P.s_rec, i, pos, mot);
+                may = may_accept(P, oj, pos, mot, P.r2_wide2);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, may);
+            cnt += __popc(m);
+            if (cnt > kFullEntries)
+                break;
+            if (may)
+                entries[cnt - __popc(m) + __popc(m & below)] = make_int2(i, k);
+        }
+        __syncwarp();
+        // exact tests, accepted samples compacted in order
+        int nacc = 0;
+        unsigned leaves = 0;
+        if (cnt <= kFullEntries)
+            for (int eb = 0; eb < cnt; eb += 32)
+            {
+                const int2 en = eb + lane < cnt ? entries[eb + lane] : make_int2(0, 0);
+                RSample r;
+                bool ok = false;
+                if (eb + lane < cnt)
+                {
+                    ok = reproject(P, en.x, oj, r.x, r.y) <= R2;
+                    r.index = en.x;
+                    r.rpos = (r.x - oj.x >= 0 ? 1 : 4) | (r.y - oj.y >= 0 ? 2 : 8);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, ok);
+                __syncwarp();
+                if (ok)
+                {
+                    const int e = nacc + __popc(m & below);
+                    T.rs[e] = r;
+                    T.leaf_of[e] = (unsigned char)en.y;
+                    leaves |= 1u << en.y;
+                }
+                nacc += __popc(m);
+                __syncwarp();
+            }
+        if (nacc == 0)
+        {
+            onward |= 1u << j;
+            continue;
+        }
+        // leaves that open a surface (RO.cpp:465-470)
+        leaves = __reduce_or_sync(0xffffffffu, leaves);
+        int since = __ffs(leaves) - 1;
+        unsigned opens = 1u << since;
+        leaves &= leaves - 1;
+        if (leaves)
+        {
+            SurfPairs values;
+            surf_pairs(leaf, oj, RANGE, P.one, values);
+            for (int v = 0; leaves; leaves &= leaves - 1, v ^= 1)
+            {
+                const int k = __ffs(leaves) - 1;
+                ulonglong2* row = reinterpret_cast<ulonglong2*>(T.values[v]);
+                if (lane == k)
+#pragma unroll
+                    for (int a = 0; a < 4; a++)
+                        row[a] = make_ulonglong2(values.v[2 * a], values.v[2 * a + 1]);
+                __syncwarp();
+                SurfPairs cur;
+#pragma unroll
+                for (int a = 0; a < 4; a++)
+                {
+                    const ulonglong2 w = row[a];
+                    cur.v[2 * a] = w.x;
+                    cur.v[2 * a + 1] = w.y;
+                }
+                if (__any_sync(0xffffffffu, lane >= since && lane < k && !same_surface_pairs(cur, values)))
+                {
+                    opens |= 1u << k;
+                    since = k;
+                }
+            }
+        }
+        // the surfaces: sample range, first strict minimum distance, quadrants
+        int nsurf = 0, start = 0;
+        for (; opens; opens &= opens - 1, nsurf++)
+        {
+            const unsigned later = opens & (opens - 1);
+            const int end_leaf = later ? __ffs(later) - 1 : 32;
+            int size = 0, quad = 0, min_index = -1;
+            float min_dist = kF32Max;
+            for (int eb = start; eb < nacc; eb += 32)
+            {
+                const int e = eb + lane;
+                const bool in = e < nacc && T.leaf_of[e] < end_leaf;
+                unsigned dbits = 0x7f800000u;
+                int qbit = 0;
+                if (in)
+                {
+                    const RSample r = T.rs[e];
+                    dbits = __float_as_uint(len2(r.x - oj.x, r.y - oj.y));
+                    qbit = 1 << (r.rpos & 3);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                quad |= __reduce_or_sync(0xffffffffu, qbit);
+                const unsigned mbits = __reduce_min_sync(0xffffffffu, dbits);
+                if (__uint_as_float(mbits) < min_dist)
+                {
+                    min_dist = __uint_as_float(mbits);
+                    min_index = eb - start + __ffs(__ballot_sync(0xffffffffu, in && dbits == mbits)) - 1;
+                }
+                size += __popc(m);
+                if (m != 0xffffffffu)
+                    break;
+            }
+            if (lane == 0)
+            {
+                Surf& sf = T.surf[nsurf];
+                sf.start = start; sf.n = size; sf.minDist = min_dist; sf.minIndex = min_index; sf.quad = quad;
+            }
+            start += size;
+        }
+        __syncwarp();
+        coop_resolve(P, oj, P.disp0, true, T.rs, T.surf, nsurf, T.tri, qcol, qidj);
+        __syncwarp();
+    }
+    warp_append(next, next_count, (onward >> lane) & 1u, entry);
+}
+
+__global__ void __launch_bounds__(kBlock, kFullBlocksPerSM)
+k_query_full(QParams P, const int* __restrict__ queue, const int* __restrict__ queue_count, float4* __restrict__ qcol,
+             int* __restrict__ next, int* __restrict__ next_count)
+{
+    __shared__ FullShared sh[kBlock / 32];
+    const int warp = (blockIdx.x * kBlock + threadIdx.x) >> 5, nwarps = gridDim.x * (kBlock / 32);
+    const int n = *queue_count;
+    const int per = entries_per_warp(n, nwarps);
+    for (long long b = (long long)warp * per; b < n; b += (long long)nwarps * per)
+        full_unit(P, queue, n, b, per, qcol, next, next_count, sh[threadIdx.x >> 5]);
 }
 
 // One warp: the queued output samples queue[b .. b+per_warp) (of n) through the full
@@ -2017,115 +2373,7 @@ __device__ __forceinline__ void coop_group(const QParams& P, const int* __restri
                 __syncwarp();
                 continue;
             }
-            // tiny-surface merging (RO.cpp:137-156): dst.samples += src.samples
-            for (int sidx = 0; fetch2R && sidx < nsurf - 1; sidx++)
-            {
-                Surf src = S.surf[sidx], dst = S.surf[sidx + 1];
-                __syncwarp();
-                if (src.n < 4)
-                {
-                    const int lo = src.start, mid = src.start + src.n, hi = dst.start + dst.n;
-                    if (src.n > 0 && mid == dst.start)
-                    {
-                        coop_reverse(S.rs, lo, mid);
-                        coop_reverse(S.rs, mid, hi);
-                        coop_reverse(S.rs, lo, hi);
-                    }
-                    if (lane == 0)
-                    {
-                        Surf& d = S.surf[sidx + 1];
-                        d.start = lo;
-                        d.n = hi - lo;
-                        if (src.minDist < dst.minDist)
-                        {
-                            d.minDist = src.minDist;
-                            d.minIndex = src.minIndex;
-                        }
-                        S.surf[sidx].n = 0;
-                    }
-                    __syncwarp();
-                }
-            }
-            // resolve (RO.cpp:165-304)
-            bool found = false;
-            float4 res = make_float4(0, 0, 0, 0);
-            float nearestDist = kF32Max;
-            int nearS = -1, nearI = 1;
-            for (int sidx = 0; sidx < nsurf && !found; sidx++)
-            {
-                const Surf sf = S.surf[sidx];
-                const int cnt = sf.n;
-                if (cnt == 0)
-                    continue;
-                const RSample* in = S.rs + sf.start;
-                if (sf.minDist < nearestDist)
-                {
-                    nearestDist = sf.minDist;
-                    nearS = sidx; nearI = sf.minIndex;
-                }
-                if (!fetch2R || sf.minDist < 0.f || sidx == nsurf - 1)
-                    found = true;
-                if (cnt >= kTriMax)
-                    found = true;
-                if (!found && cnt >= 3)
-                    found = coop_triangle(in, cnt, o, dispersion, T);
-                if (found)
-                {
-                    // tent filter (RO.cpp:274-294): products in parallel, summed
-                    // in sample order by every lane from shuffles
-                    res = make_float4(0, 0, 0, 0);
-                    for (int kb = 0; kb < cnt; kb += 32)
-                    {
-                        const int k = kb + lane;
-                        float4 pr = make_float4(0, 0, 0, 0);
-                        bool inc = false;
-                        if (k < cnt)
-                        {
-                            const RSample r = in[k];
-                            const float dx = o.x - r.x, dy = o.y - r.y;
-                            const float weight = 1 - len2(dx, dy) / dispersion;
-                            if (weight > 0)
-                            {
-                                const float4 c = P.s_col[r.index];
-                                pr = make_float4(c.x * weight, c.y * weight, c.z * weight, c.w * weight);
-                                inc = true;
-                            }
-                        }
-                        for (unsigned mi = __ballot_sync(0xffffffffu, inc); mi; mi &= mi - 1)
-                        {
-                            const int src = __ffs(mi) - 1;
-                            res.x += __shfl_sync(0xffffffffu, pr.x, src);
-                            res.y += __shfl_sync(0xffffffffu, pr.y, src);
-                            res.z += __shfl_sync(0xffffffffu, pr.z, src);
-                            res.w += __shfl_sync(0xffffffffu, pr.w, src);
-                        }
-                    }
-                    const float oow = rcp(res.w);
-                    res.x *= oow; res.y *= oow; res.z *= oow; res.w *= oow;
-                    nearS = sidx; nearI = sf.minIndex;
-                }
-            }
-            if (lane == 0)
-            {
-                float4 out = make_float4(0, 0, 0, 0);
-                if (nearS != -1)
-                {
-                    if (res.w == 0)
-                        res = P.s_col[S.rs[S.surf[nearS].start + nearI].index];
-                    if (P.lens_filter == 1)
-                    {
-                        float g = gaussian(o.u, 0.5f, 0) * gaussian(o.v, 0.5f, 0);
-                        res.x *= g; res.y *= g; res.z *= g; res.w *= g;
-                    }
-                    if (P.time_filter == 1)
-                    {
-                        float g = gaussian(o.t, 0.25f, 0.5f);
-                        res.x *= g; res.y *= g; res.z *= g; res.w *= g;
-                    }
-                    out = res;
-                }
-                qcol[qj] = out;
-            }
+            coop_resolve(P, o, dispersion, fetch2R, S.rs, S.surf, nsurf, T, qcol, qj);
             __syncwarp();
         }
         todo = redo;
@@ -3058,9 +3306,12 @@ void accept_bound(QParams& P, const Ctx& c, const float* uvt)
     const double most_coc = 512.0;      // |C0| / w beyond which a sample is always tested exactly
     P.min_w = (float)std::max(std::fabs((double)P.c0) / most_coc, 1e-30);
     const double D = U * (most_coc * 1.001 + std::fabs((double)P.c1));
-    const double m = 1.5 * e * (64.0 * X + 20.0 * O + 36.0 * D + 24.0 * R);
-    const double r = R * (1.0 + 8.0 * e) + 1.5 * m;
-    P.r2_wide = (float)(r * r * (1.0 + 8.0 * e));
+    for (int k = 1; k <= 2; k++)
+    {
+        const double m = 1.5 * e * (64.0 * X + 20.0 * O + 36.0 * D + 24.0 * k * R);
+        const double r = k * R * (1.0 + 8.0 * e) + 1.5 * m;
+        (k == 1 ? P.r2_wide : P.r2_wide2) = (float)(r * r * (1.0 + 8.0 * e));
+    }
 }
 
 QParams make_params(const Ctx& c)
@@ -3159,6 +3410,7 @@ int light_default_blocks(const Ctx& c)
 // run one after another in the graph, reusing it.  The light pass's tile shape
 // is chosen per frame by timing each shape (autotune).
 // ---------------------------------------------------------------------------
+constexpr int kFrameCounters = 5;
 struct FrameDesc
 {
     QParams P;
@@ -3168,7 +3420,7 @@ struct FrameDesc
     float4* qcol;
     int* heavy;
     int* ovf;
-    int* counters;          // [0] overflow queue, [1] capacity failures, [2] heavy queue, [3] retry list
+    int* counters;          // [0] overflow queue, [1] capacity failures, [2] heavy queue, [3] retry list, [4] cooperative pass
     float4* out;
 };
 
@@ -3241,7 +3493,8 @@ k_batch_light(const FrameDesc* __restrict__ fd, const long long* __restrict__ un
 
 // Work items of a pass over the frames' queues (counters[which]; 3: the retry
 // lists, 2: the full path): per_warp entries per warp, which is stored behind
-// the items' frame offsets.  warps_per_item: 4 for the retry pass's blocks.
+// the items' frame offsets (which = 4: the cooperative pass).  warps_per_item: 4
+// for the retry pass's blocks.
 __global__ void __launch_bounds__(32)
 k_batch_items(const FrameDesc* __restrict__ fd, int nframes, int which, int warps_per_item, int nwarps,
               long long* __restrict__ item_begin)
@@ -3275,6 +3528,30 @@ k_batch_items(const FrameDesc* __restrict__ fd, int nframes, int which, int warp
     }
 }
 
+// The full path's first kernel over every frame of a chunk: a warp takes one item at a time.
+__global__ void __launch_bounds__(kBlock, kFullBlocksPerSM)
+k_batch_full(const FrameDesc* __restrict__ fd, const long long* __restrict__ item_begin, int nframes,
+             unsigned long long* __restrict__ next_item)
+{
+    __shared__ FullShared sh[kBlock / 32];
+    const int lane = threadIdx.x & 31;
+    const long long total = item_begin[nframes];
+    const int per = (int)item_begin[nframes + 1];
+    for (;;)
+    {
+        long long it = 0;
+        if (lane == 0)
+            it = (long long)atomicAdd(next_item, 1ull);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= total)
+            break;
+        const int f = frame_of(item_begin, nframes, it);
+        const FrameDesc& D = fd[f];
+        full_unit(D.P, D.heavy, D.counters[2], (it - item_begin[f]) * per, per, D.qcol, D.ovf, D.counters + 4,
+                  sh[threadIdx.x >> 5]);
+    }
+}
+
 // Full-path pass over every frame of a chunk: a warp takes one item at a time.
 __global__ void __launch_bounds__(kCWarps * 32, TLFR_COOP_BLOCKS_PER_SM)
 k_batch_coop(const FrameDesc* __restrict__ fd, const long long* __restrict__ item_begin, int nframes,
@@ -3295,7 +3572,7 @@ k_batch_coop(const FrameDesc* __restrict__ fd, const long long* __restrict__ ite
             break;
         const int f = frame_of(item_begin, nframes, it);
         const FrameDesc& D = fd[f];
-        coop_group(D.P, D.heavy, D.counters[2], (int)(it - item_begin[f]) * per, D.qcol, D.ovf, D.counters + 0,
+        coop_group(D.P, D.ovf, D.counters[4], (int)(it - item_begin[f]) * per, D.qcol, D.heavy, D.counters + 0,
                    (int)D.nq, scratch[warp], sh_tri[threadIdx.x >> 5], per);
     }
 }
@@ -3334,7 +3611,7 @@ struct BatchChunk
     long long* d_item_begin = nullptr;  // count + 2 (k_batch_items)
     long long* d_pix_begin = nullptr;   // count + 1
     long long* d_retry_begin = nullptr; // count + 2
-    unsigned long long* d_work = nullptr;   // [0] next light unit, [1] next full-path item, [2] next retry unit
+    unsigned long long* d_work = nullptr;   // [0] next light unit, [1] next cooperative item, [2] next retry unit, [3] next full-path item
 };
 
 struct BatchPlan
@@ -3347,7 +3624,7 @@ struct BatchPlan
     FrameDesc* d_desc = nullptr;
     long long* d_offsets = nullptr;
     unsigned long long* d_work = nullptr;
-    int* d_counters = nullptr;          // 4 per frame
+    int* d_counters = nullptr;          // kFrameCounters per frame
     float4* qcol = nullptr;
     int* heavy = nullptr;
     int* ovf = nullptr;
@@ -3388,7 +3665,7 @@ static tlfr_status light_trial(const FrameDesc& D, const Ctx& c, int shape, cuda
         L.units = std::max<long long>(std::min<long long>(L.units, 4096), L.units / 8);
     }
     const int blocks = (int)std::min<long long>(L.units, (long long)c.num_sms * 64);
-    CKB(cudaMemsetAsync(D.counters, 0, 4 * sizeof(int), s));
+    CKB(cudaMemsetAsync(D.counters, 0, kFrameCounters * sizeof(int), s));
     CKB(cudaEventRecord(e0, s));
     K_LIGHT_PLAIN(false)<<<blocks, kBlock, 0, s>>>(D.P, L, D.nq, D.qcol, D.heavy, D.counters + 2, nullptr, nullptr);
     CKB(cudaEventRecord(e1, s));
@@ -3478,7 +3755,7 @@ tlfr_status batch_build(BatchPlan& bp, const std::vector<BatchEntry>& entries, c
     CKB(cudaMalloc(&bp.qcol, sizeof(float4) * cap));
     CKB(cudaMalloc(&bp.heavy, sizeof(int) * cap));
     CKB(cudaMalloc(&bp.ovf, sizeof(int) * cap));
-    CKB(cudaMalloc(&bp.d_counters, sizeof(int) * 4 * n));
+    CKB(cudaMalloc(&bp.d_counters, sizeof(int) * kFrameCounters * n));
     CKB(cudaMalloc(&bp.coop_scratch, coop_scratch_bytes(bp.num_sms)));
     CKB(cudaMalloc(&bp.ovf_scratch, overflow_scratch_bytes()));
     for (const BatchChunk& ch : bp.chunks)
@@ -3490,7 +3767,7 @@ tlfr_status batch_build(BatchPlan& bp, const std::vector<BatchEntry>& entries, c
             D.qcol = bp.qcol + off;
             D.heavy = bp.heavy + off;
             D.ovf = bp.ovf + off;
-            D.counters = bp.d_counters + 4 * f;
+            D.counters = bp.d_counters + kFrameCounters * f;
             off += nq[f];
         }
     }
@@ -3547,14 +3824,14 @@ tlfr_status batch_build(BatchPlan& bp, const std::vector<BatchEntry>& entries, c
     // device tables
     CKB(cudaMalloc(&bp.d_desc, sizeof(FrameDesc) * n));
     CKB(cudaMalloc(&bp.d_offsets, sizeof(long long) * (4 * n + 6 * bp.chunks.size())));
-    CKB(cudaMalloc(&bp.d_work, sizeof(unsigned long long) * 3 * bp.chunks.size()));
+    CKB(cudaMalloc(&bp.d_work, sizeof(unsigned long long) * 4 * bp.chunks.size()));
     std::vector<long long> offs;
     offs.reserve(4 * n + 6 * bp.chunks.size());
     for (size_t k = 0; k < bp.chunks.size(); k++)
     {
         BatchChunk& ch = bp.chunks[k];
         ch.d_desc = bp.d_desc + ch.first;
-        ch.d_work = bp.d_work + 3 * k;
+        ch.d_work = bp.d_work + 4 * k;
         const size_t base = offs.size();
         long long u = 0, pxl = 0;
         std::vector<long long> ub, pb;
@@ -3586,8 +3863,8 @@ tlfr_status batch_enqueue(BatchPlan& bp, cudaStream_t s, std::string& err, long 
 {
     const int n = (int)bp.entries.size();
     long long L = 0;
-    CKB(cudaMemsetAsync(bp.d_counters, 0, sizeof(int) * 4 * n, s));
-    CKB(cudaMemsetAsync(bp.d_work, 0, sizeof(unsigned long long) * 3 * bp.chunks.size(), s));
+    CKB(cudaMemsetAsync(bp.d_counters, 0, sizeof(int) * kFrameCounters * n, s));
+    CKB(cudaMemsetAsync(bp.d_work, 0, sizeof(unsigned long long) * 4 * bp.chunks.size(), s));
     for (const BatchChunk& ch : bp.chunks)
     {
         // the router's flags for this chunk's routed frames (their descriptors
@@ -3618,16 +3895,20 @@ tlfr_status batch_enqueue(BatchPlan& bp, cudaStream_t s, std::string& err, long 
                                        ch.d_retry_begin);
         k_batch_light<false><<<bp.num_sms * kL2BlocksPerSM, kBlock, 0, s>>>(ch.d_desc, ch.d_retry_begin, ch.count,
                                                                           ch.d_work + 2);
-        k_batch_items<<<1, 32, 0, s>>>(ch.d_desc, ch.count, 2, 1, bp.num_sms * kCoopBlocksPerSM * kCWarps,
+        k_batch_items<<<1, 32, 0, s>>>(ch.d_desc, ch.count, 2, 1, bp.num_sms * kFullBlocksPerSM * (kBlock / 32),
+                                       ch.d_item_begin);
+        k_batch_full<<<bp.num_sms * kFullBlocksPerSM, kBlock, 0, s>>>(ch.d_desc, ch.d_item_begin, ch.count,
+                                                                     ch.d_work + 3);
+        k_batch_items<<<1, 32, 0, s>>>(ch.d_desc, ch.count, 4, 1, bp.num_sms * kCoopBlocksPerSM * kCWarps,
                                        ch.d_item_begin);
         k_batch_coop<<<bp.num_sms * kCoopBlocksPerSM, kCWarps * 32, 0, s>>>(ch.d_desc, ch.d_item_begin, ch.count,
                                                                            ch.d_work + 1,
                                                                            reinterpret_cast<CoopScratch*>(bp.coop_scratch));
-        L += 5;
+        L += 7;
         for (int f = ch.first; f < ch.first + ch.count; f++)
         {
             const FrameDesc& D = bp.desc[f];
-            k_query_overflow<<<kOvSlots / 64, 64, 0, s>>>(D.P, D.ovf, D.counters + 0, (int)D.nq, D.qcol,
+            k_query_overflow<<<kOvSlots / 64, 64, 0, s>>>(D.P, D.heavy, D.counters + 0, (int)D.nq, D.qcol,
                                                          (char*)bp.ovf_scratch,
                                                          slot_bytes_for(kOvStack, kOvLeaf, kOvRs, kOvSurf), kOvSlots,
                                                          kOvStack, kOvLeaf, kOvRs, kOvSurf, D.counters + 1, nullptr, 0);
@@ -3669,12 +3950,12 @@ void batch_info(const BatchPlan& bp, int* shapes, int* chunks)
 tlfr_status batch_failures(BatchPlan& bp, cudaStream_t s, std::vector<int>& hard, std::string& err)
 {
     const int n = (int)bp.entries.size();
-    std::vector<int> cnt(4 * n);
-    CKB(cudaMemcpyAsync(cnt.data(), bp.d_counters, sizeof(int) * 4 * n, cudaMemcpyDeviceToHost, s));
+    std::vector<int> cnt(kFrameCounters * n);
+    CKB(cudaMemcpyAsync(cnt.data(), bp.d_counters, sizeof(int) * kFrameCounters * n, cudaMemcpyDeviceToHost, s));
     CKB(cudaStreamSynchronize(s));
     hard.resize(n);
     for (int f = 0; f < n; f++)
-        hard[f] = cnt[4 * f + 1] + (cnt[4 * f + 0] > (int)bp.desc[f].nq ? 1 : 0);
+        hard[f] = cnt[kFrameCounters * f + 1] + (cnt[kFrameCounters * f + 0] > (int)bp.desc[f].nq ? 1 : 0);
     return TLFR_OK;
 }
 
@@ -3778,7 +4059,7 @@ tlfr_status reconstruct_frame(Ctx& c, float4* d_rgba, bool collect_stats)
         return fb;
     if (c.params.enable_cuda)
         return reconstruct_toggle(c, d_rgba);
-    int* counters = reinterpret_cast<int*>(c.d_stats + 1);   // [0] overflow, [1] hard, [2] heavy, [3] retry
+    int* counters = reinterpret_cast<int*>(c.d_stats + 1);   // [0] overflow, [1] hard, [2] heavy, [3] retry, [4] cooperative
     QParams P = make_params(c);
     CKQ(cudaMemsetAsync(c.d_stats, 0, sizeof(DevStats) + 8 * sizeof(int), s));
     if ((c.router || c.route_all_fast) && !c.route_prob)
@@ -3839,8 +4120,12 @@ tlfr_status reconstruct_frame(Ctx& c, float4* d_rgba, bool collect_stats)
         TLFR_LAUNCH(c, K_LIGHT_RETRY, c.num_sms * kL2BlocksPerSM, kBlock, s, P, light_map(c), nq, c.qcol,
                     c.heavy_queue, counters + 2, c.ovf_queue, counters + 3);
         CKQ(cudaEventRecord(c.evq1, s));
-        TLFR_LAUNCH(c, k_query_coop, coop_blocks(c), kCWarps * 32, s, P, c.heavy_queue, counters + 2, c.qcol,
-                    c.ovf_queue, counters + 0, (int)c.ovf_cap, reinterpret_cast<CoopScratch*>(c.coop_scratch));
+        // the queue's output samples that need more go to the overflow queue (the
+        // retry pass has read it), and what outgrows that to the first queue
+        TLFR_LAUNCH(c, k_query_full, c.num_sms * kFullBlocksPerSM, kBlock, s, P, c.heavy_queue, counters + 2, c.qcol,
+                    c.ovf_queue, counters + 4);
+        TLFR_LAUNCH(c, k_query_coop, coop_blocks(c), kCWarps * 32, s, P, c.ovf_queue, counters + 4, c.qcol,
+                    c.heavy_queue, counters + 0, (int)c.ovf_cap, reinterpret_cast<CoopScratch*>(c.coop_scratch));
     }
     CKQ(cudaEventRecord(c.evq2, s));
     CKQ(cudaGetLastError());
@@ -3865,7 +4150,8 @@ tlfr_status reconstruct_frame(Ctx& c, float4* d_rgba, bool collect_stats)
             CKQ(cudaMalloc(&c.ovf_scratch, c.ovf_scratch_bytes));
         }
         const int slots = std::min(kOvSlots, novf);
-        TLFR_LAUNCH(c, k_query_overflow, (slots + 63) / 64, 64, s, P, c.ovf_queue, counters + 0, (int)c.ovf_cap,
+        TLFR_LAUNCH(c, k_query_overflow, (slots + 63) / 64, 64, s, P, collect_stats ? c.ovf_queue : c.heavy_queue,
+                    counters + 0, (int)c.ovf_cap,
                     c.qcol, (char*)c.ovf_scratch,
                     sb, slots, kOvStack, kOvLeaf, kOvRs, kOvSurf, counters + 1, c.d_stats, collect_stats ? 1 : 0);
         CKQ(cudaGetLastError());
