@@ -14,12 +14,14 @@
 // nothing was found (Reconstruction.cpp:649-720).
 //
 // The work runs in passes:
-//   k_query_light     every output sample: each lane collects its own leaves at
-//                     1R into shared memory, then the warp scans each lane's
-//                     sample in turn; settles the samples the 1R fetch settles
-//                     (fetch2R false) and queues the rest
-//   k_query_coop      the queue, warp-cooperatively: the full path from the 2R
-//                     fetch (or from 1R for samples that outgrew the light pass)
+//   k_query_light     every output sample: each collects its leaves at 1R into
+//                     shared memory, then the warp scans them in turn; settles the
+//                     samples the 1R fetch settles (fetch2R false) and queues the
+//                     rest; a second launch retries those that outgrow the first
+//   k_query_full      the queue, in the same way at 2R: the full path of output
+//                     samples whose 2R fetch fits the kernel's lists
+//   k_query_coop      the rest, warp-cooperatively: the full path from the 2R fetch
+//                     (or from 1R for samples that outgrew the light pass)
 //   k_query_overflow  the few samples that outgrow the cooperative pass's lists,
 //                     with large capacities from a global arena; a sample that
 //                     outgrows those too is reported as TLFR_OVERFLOW
@@ -1177,8 +1179,10 @@ __device__ __forceinline__ bool light_query_id(const QParams& P, const LightMap&
 //   4. lanes over (output sample, colour component): the tent filter summed in
 //      acceptance order (RO.cpp:274-294), four colours loaded at a time, and the
 //      nearest sample.
-// 1920x1080x8, both tiers: LIGHT_NOW ms; with every chunk's samples reprojected exactly
-// and handled leaf by leaf with their colours loaded and shuffled: 934 ms.
+// 1920x1080x8, both tiers: 755 ms; with every chunk's samples reprojected exactly
+// and handled leaf by leaf, their colours loaded and shuffled: 934 ms.  First tier
+// at 960x540x8: 137.8 ms, 103 G warp instructions, 66% issue active, 67% of the L1
+// wavefronts' peak; before, 195.5 ms, 165 G, 74%, 72%.
 template <bool PROBE, int LEAF, int STACK, int MODE>
 __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, long long u, long long num_queries,
                                            float4* __restrict__ qcol, int* __restrict__ heavy,
