@@ -1245,6 +1245,7 @@ __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, 
     const float RANGE = 1.0f / sqrtf(128.0f);
     const float* colours = reinterpret_cast<const float*>(P.s_col);
     int cnt = 0, nslot = 0;         // samples set aside, slots in use
+    int live = 0;                   // slots before it are finished
     // lane -> (slot, colour component) and that slot's running surface state
     const int my_slot = lane >> 2, comp = lane & 3;
     int e0 = 0, e1 = 0, my_j = 0;   // the slot's samples set aside, its output sample's lane
@@ -1350,7 +1351,7 @@ __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, 
                 }
             }
             // finished output samples
-            const bool fin = my_slot < nslot && !(open && my_slot == nslot - 1);
+            const bool fin = my_slot >= live && my_slot < nslot && !(open && my_slot == nslot - 1);
             const int seen = T.seen[my_slot];
             const bool redo = MODE == kLightFirst && (seen & 32);
             const bool settled = T.first_leaf[my_slot] < 32 && (seen < 16 || (seen & 15) == 15 || ((fast_lanes >> my_j) & 1u)) && !redo;
@@ -1385,6 +1386,7 @@ __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, 
             e0 = e1 = 0;
             if (!open)
                 nslot = 0;
+            live = open ? nslot - 1 : 0;
             if (!todo)
                 break;
         }

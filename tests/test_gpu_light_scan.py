@@ -56,6 +56,10 @@ def test_light_scan_edges_match_oracle(kind, opt):
     img = g.reconstructDofMotion()
     ref = CpuRecon("orc", rec, coc, **opt).reconstruct()
     assert np.array_equal(img.view(np.uint32), ref.view(np.uint32))
+    # an output sample is queued for the full path once, also when the scan's list
+    # fills up inside another one of its warp (the queue holds one entry for each)
+    outputs = img.shape[0] * img.shape[1] * (1 if p.overrideUVT else p.outputSpp or 128)
+    assert g.stats().num_heavy_queries <= outputs
 
 
 @pytest.mark.parametrize("seed", [6, 1235])
