@@ -1012,9 +1012,11 @@ __device__ __forceinline__ float reproject(const QParams& P, int i, const Query&
 // Whether a sample may lie within the radius whose widened square is r2w
 // (accept_bound()): the reprojection with fused multiply-adds and the
 // hardware's reciprocal (relative error at most 2^-23) in place of two exact
-// divisions, about 17 instructions against 50.  Never false for a sample that
+// divisions, about 18 instructions against 50.  Never false for a sample that
 // reproject() puts within the radius.  Samples whose w at the output time is
-// outside the range the bound is derived for always may.
+// outside the range the bound is derived for always may: near ones, and those
+// beyond kMaxW, whose reciprocal is subnormal and comes back as zero.
+constexpr float kMaxW = 8e37f;      // below 2^126
 __device__ __forceinline__ bool may_accept(const QParams& P, const Query& o, const float4& sp4, const float4& sm,
                                            float r2w)
 {
@@ -1028,7 +1030,7 @@ __device__ __forceinline__ bool may_accept(const QParams& P, const Query& o, con
     const float dx = __fmaf_rn(o.u, coc, __fmaf_rn(Px, r, -o.x));
     const float dy = __fmaf_rn(o.v, coc, __fmaf_rn(Py, r, -o.y));
     const float d2 = __fmaf_rn(dx, dx, dy * dy);
-    return !(d2 > r2w) || !(Pw >= fmaxf(0.5f * sp4.z, P.min_w));
+    return !(d2 > r2w) || !(Pw >= fmaxf(0.5f * sp4.z, P.min_w) && Pw <= kMaxW);
 }
 
 __device__ __forceinline__ Query query_of(const QParams& P, long long q)
@@ -3299,7 +3301,7 @@ size_t slot_bytes_for(int stack_cap, int leaf_cap, int rs_cap, int surf_cap)
 // Bounds of may_accept() for a hierarchy and output setting (uvt: the override,
 // or null for the pattern, whose |u|, |v| are at most 1).  With e = 2^-24,
 // X the largest sample coordinate, O the largest output coordinate, |u|, |v| <= U,
-// w >= max(z / 2, min_w) and so D = U (|C0| / min_w + |C1|) the largest CoC term:
+// kMaxW >= w >= max(z / 2, min_w) and so D = U (|C0| / min_w + |C1|) the largest CoC term:
 // of a sample within the radius, both reprojections are within
 // (15 (|x z| + |m dt|) / w + 16 D + 3 R + 2 O) e of the real one between them, and
 // (|x z| + |m dt|) / w <= 4 X + O + D + R.  Widened by half again.
