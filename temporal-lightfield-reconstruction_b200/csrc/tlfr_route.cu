@@ -385,10 +385,11 @@ k_mlp_train(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Wh, c
 {
     static_assert(kTrainWarps * 16 == kH, "a warp owns 16 rows of the weight gradients");
     __shared__ float s_grad[kNumTrain];
-    __shared__ __nv_bfloat16 s_h1[kTrainWarps][16][kH];
-    __shared__ __nv_bfloat16 s_dh2[kTrainWarps][16][kH];
-    __shared__ __nv_bfloat16 s_dh1[kTrainWarps][16][kH];
-    __shared__ __nv_bfloat16 s_x[kTrainWarps][16][kF];
+    // written two values at a time
+    __shared__ alignas(4) __nv_bfloat16 s_h1[kTrainWarps][16][kH];
+    __shared__ alignas(4) __nv_bfloat16 s_dh2[kTrainWarps][16][kH];
+    __shared__ alignas(4) __nv_bfloat16 s_dh1[kTrainWarps][16][kH];
+    __shared__ alignas(4) __nv_bfloat16 s_x[kTrainWarps][16][kF];
     __shared__ float s_loss;
     for (int i = threadIdx.x; i < kNumTrain; i += blockDim.x)
         s_grad[i] = 0.0f;
