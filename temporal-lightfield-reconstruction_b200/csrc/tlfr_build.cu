@@ -27,6 +27,7 @@
 #include "tlfr_internal.h"
 
 #include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <cstring>
 
@@ -963,41 +964,28 @@ __device__ int emit_nodes(bool is_root, BNode* f, int size, QNode* nodes, float2
     const int lim = is_root ? 1 : 4;
     while (size > lim)
     {
-        float best = kF32Max;
-        unsigned at = 0xffffffffu;      // i << 16 | j
-        for (int p = lane, i = 0, row = 0;; p += G)
+        float mine = kF32Max;
+        int ci = INT_MAX, cj = INT_MAX;
+        for (PairWalk p(size, lane); !p.done(); p.advance(G))
         {
-            // pair p: rows of i against j > i; row = pairs before row i
-            while (i < size - 1 && p >= row + size - 1 - i)
-            {
-                row += size - 1 - i;
-                i++;
-            }
-            if (i >= size - 1)
-                break;
-            const int j = i + 1 + (p - row);
-            const BNode n0 = f[i], n1 = f[j];
+            const BNode n0 = f[p.i], n1 = f[p.j];
             BNode m;
             node_merge(n0, n1, m);
             const float cost = bnode_cost(m) - (bnode_cost(n0) + bnode_cost(n1));
-            if (cost < best)
+            if (cost < mine)
             {
-                best = cost;
-                at = (unsigned)i << 16 | (unsigned)j;
+                mine = cost;
+                ci = p.i;
+                cj = p.j;
             }
         }
+        float best = mine;
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1)
-        {
-            const float ob = __shfl_xor_sync(group, best, o);
-            const unsigned oa = __shfl_xor_sync(group, at, o);
-            if (ob < best || (ob == best && oa < at))
-            {
-                best = ob;
-                at = oa;
-            }
-        }
-        const int mi = at == 0xffffffffu ? 0 : (int)(at >> 16), mj = at == 0xffffffffu ? 1 : (int)(at & 0xffffu);
+            best = fminf(best, __shfl_xor_sync(group, best, o));
+        int mi = __reduce_min_sync(group, mine == best ? ci : INT_MAX);
+        int mj = __reduce_min_sync(group, mine == best && ci == mi ? cj : INT_MAX);
+        if (mi == INT_MAX) { mi = 0; mj = 1; }
         if (lane == 0)
         {
             const BNode n0 = f[mi], n1 = f[mj];

@@ -337,6 +337,24 @@ TLFR_HD void fw_sort(A& a, int start, int end)
     }
 }
 
+// Pairs (i, j), i < j, of size items in the order of i, then j: the first-th pair,
+// and on by n at a time.  Past the last pair i == size - 1.
+struct PairWalk
+{
+    int size, i, j;
+    TLFR_HD PairWalk(int size, int first) : size(size), i(0), j(1) { advance(first); }
+    TLFR_HD bool done() const { return i >= size - 1; }
+    TLFR_HD void advance(int n)
+    {
+        j += n;
+        while (!done() && j >= size)
+        {
+            i++;
+            j = i + 1 + (j - size);
+        }
+    }
+};
+
 // Jenkins hash hashBits(a, b) (framework/base/Hash.hpp:169-183)
 TLFR_HD uint32_t hash_bits(uint32_t a, uint32_t b)
 {
