@@ -38,3 +38,20 @@ def test_feature_rows_at_any_float(offset):
         router.close()
     for a, b in zip(*got):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,repeat", [(100003, 1), (1 << 18, 1), (1 << 18, 16)])
+def test_gradient_of_many_rows(n, repeat):
+    """Several groups of rows per block, against the BF16 network in 64 bits.  Repeating
+    the rows a power of two times changes no rounding but that of the sums.  Bound: an
+    accumulator goes through 32 truncating mma, each losing half a unit in the last place
+    of a sum that grows to its end (32 * 2^-24 / 2, 1e-6), and 5e-7 for the sums in FP32
+    and for activations that round to BF16 the other way (1/sqrt(n))."""
+    torch, feats, labels = _rows(n, 7)
+    router = tlfr.Router(0, seed=11, mean=np.full(R.F, 1, np.float32), inv_std=np.full(R.F, 0.5, np.float32))
+    f, y = feats.repeat(repeat, 1), labels.repeat(repeat)
+    torch.cuda.synchronize()
+    grad, _ = router.gradient(f.data_ptr(), y.data_ptr(), n * repeat)
+    want = R.gradient(router.params(), feats.cpu().numpy(), labels.cpu().numpy())
+    router.close()
+    assert np.linalg.norm(grad - want) <= 1.5e-6 * np.linalg.norm(want)
