@@ -19,7 +19,7 @@
 //   k_leaf_scan       surface scan and leaf nodes (RTB.cpp:222-378)
 //   k_emit_level      emitNodes at every kd node inside a task, deepest level first
 //                     (RTB.cpp:384-451)
-//   k_top             serial top of the tree (Reconstruction.cpp:192-203)
+//   k_top             the tasks' frontiers merged in pairs, and the root (Reconstruction.cpp:192-203)
 //
 // Node indices differ from the reference's (nodes are emitted in parallel), the
 // tree structure, the child order, every bound and the sample order do not.
@@ -41,7 +41,7 @@ constexpr int kMaxKdLevels = 40;
 constexpr int kTopCap = 1 << 16;
 
 // error codes written to GridInfo::error
-enum { kErrNone = 0, kErrKdDepth = 1, kErrTopCap = 2, kErrEmpty = 3 };
+enum { kErrNone = 0, kErrTopCap = 2, kErrEmpty = 3 };
 
 __device__ __forceinline__ unsigned float_to_ordered(float f)
 {
@@ -1342,7 +1342,7 @@ tlfr_status build_hierarchy(Ctx& c, const float* d_records)
                                                           c.sbounds, c.surface, c.pending);
     CK(cudaGetLastError());
 
-    // --- emitNodes bottom-up, then the serial top ---
+    // --- emitNodes bottom-up, then the top ---
     for (int L = levels - 1; L >= 5; L--)
     {
         const size_t most = std::min<size_t>((size_t)1 << std::min(L, 30), (size_t)c.grid.num_kd) * kEmitGroup;

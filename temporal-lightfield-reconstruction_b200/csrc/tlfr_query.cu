@@ -93,8 +93,6 @@ TLFR_HD void load_sample(const float4* rec, int i, float4& pos, float4& mot)
 #endif
 }
 
-
-
 enum { kQOk = 0, kQOverflow = 1 };
 
 // Node i (64 bytes, 64-byte aligned) in two 256-bit loads.
@@ -1075,11 +1073,15 @@ __device__ __forceinline__ void warp_append(int* queue, int* count, bool pred, i
 constexpr int kQueueRestart = 1 << 30;
 
 constexpr int kProbe = 4;
-// Light-pass blocks per SM, by shared memory (24.5 KB per block of the first
-// tier, 32 KB of the others) and registers.
+// Light-pass blocks per SM that the kernels are compiled for and the persistent
+// grids of batches launched with, by shared memory (26.5 KB per block of the first
+// tier, 34.5 KB of the others) and registers.  The first tier of a single frame
+// needs 64 registers, so 8 of its blocks fit; in a batch it needs 67.
 constexpr int kProbeBlocksPerSM = 6;
 constexpr int kL1BlocksPerSM = 7;
 constexpr int kL2BlocksPerSM = 6;
+static_assert(kBlock / 32 * sizeof(LightShared<kL1Leaf, kL1Stack>) == 27136 &&
+              kBlock / 32 * sizeof(LightShared<kL2Leaf, kL2Stack>) == 35328, "the sizes above");
 // Light-pass kinds: every output sample of a map, overflow to the full path
 // (kLightPlain); the same with overflow to a retry list (kLightFirst); the
 // output samples of a retry list (kLightRetry), overflow to the full path.
@@ -1168,9 +1170,8 @@ __device__ __forceinline__ bool light_query_id(const QParams& P, const LightMap&
 // The scan is bound by instruction issue, so it does per tested sample only what
 // 93% of them need, and the rest once per batch of output samples:
 //   1. the warp runs over the output sample's leaves' samples as one flat
-//      sequence, 32 at a time across leaf boundaries (32-byte records, the next
-//      chunk on its way while the current one is tested), and sets aside those
-//      that may_accept();
+//      sequence, 32 at a time across leaf boundaries (32-byte records), and sets
+//      aside those that may_accept();
 //   2. where they come from more than one leaf, sameSurface
 //      (Reconstruction.hpp:457-525) of each such leaf with every earlier one from
 //      the first, lanes over the earlier leaves, as bit masks;
@@ -1183,7 +1184,7 @@ __device__ __forceinline__ bool light_query_id(const QParams& P, const LightMap&
 //      nearest sample.
 // 1920x1080x8, both tiers: 755 ms; with every chunk's samples reprojected exactly
 // and handled leaf by leaf, their colours loaded and shuffled: 934 ms.  First tier
-// at 960x540x8: 137.8 ms, 103 G warp instructions, 66% issue active, 67% of the L1
+// at 960x540x8: 137.4 ms, 106 G warp instructions, 68% issue active, 66% of the L1
 // wavefronts' peak; before, 195.5 ms, 165 G, 74%, 72%.
 template <bool PROBE, int LEAF, int STACK, int MODE>
 __device__ __forceinline__ void light_unit(const QParams& P, const LightMap& L, long long u, long long num_queries,
@@ -1575,9 +1576,11 @@ k_query_light(QParams P, LightMap L, long long num_queries, float4* __restrict__
 // ---------------------------------------------------------------------------
 constexpr int kCWarps = 4;
 // blocks of the cooperative full-path pass (its working lists are per warp):
-// 5 per SM leave it its 95 registers without spills; at 1920x1080x8 it measured
-// 404 ms against 512 ms at 6 (80 registers, spills; earlier 563 against 651
-// and 699 at 8 blocks)
+// 5 per SM leave it its 96 registers without spills; the full path of a
+// 1920x1080x8 frame (k_query_full before it) takes 426 ms against 455 at 6 (80
+// registers, spills) and 438 at 4.  At 960x540x8 it takes 37.4 ms for the 3 M
+// entries passed on: long scoreboard 5.1 and no instruction 3.7 stalls per issue,
+// 34% issue active (its instruction footprint)
 #ifndef TLFR_COOP_BLOCKS_PER_SM
 #define TLFR_COOP_BLOCKS_PER_SM 5
 #endif
@@ -1842,8 +1845,6 @@ __device__ __forceinline__ void coop_reverse(RSample* a, int lo, int hi)     // 
 // beyond k that complete the quadrants (bit masks per quadrant pattern) and the
 // within-dispersion condition (a bit mask), each checked against k's side
 // length before the edge functions.
-
-
 __device__ bool coop_triangle(const RSample* in, int n, const Query& o, float dispersion, TriShared& T)
 {
     const int lane = threadIdx.x & 31;
@@ -2069,6 +2070,9 @@ __device__ __forceinline__ void coop_resolve(const QParams& P, const Query& o, f
 // and scan at 2R, with the lists of one output sample at a time in shared memory;
 // the accepted samples are compacted in order, and surfaces open where a leaf is
 // not one surface with a leaf since the open one began (RO.cpp:412-503).
+// Passed on: 3% of the queue at 962x543x4, 25% at 1920x1080x8, 41% at 960x540x8
+// (another seed), whose 2R fetches reach more than 32 leaves.  Issue and latency:
+// 57% issue active, stalls long scoreboard 2.5, wait 2.6, short scoreboard 1.4.
 // ---------------------------------------------------------------------------
 constexpr int kFullLeaf = 32, kFullStack = 32, kFullEntries = 192;
 constexpr int kFullBlocksPerSM = 6;
@@ -3660,7 +3664,8 @@ void batch_release(BatchPlan& bp)
 #define CKB(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { err = std::string(#x) + ": " + cudaGetErrorString(_e); return (_e == cudaErrorMemoryAllocation) ? TLFR_OOM : TLFR_CUDA; } } while (0)
 
 // The light pass of one frame alone with a given tile shape (autotune), over
-// its first eighth of block iterations (the top rows of the frame's tiles).
+// its first eighth of block iterations (the top rows of the frame's tiles), in
+// the form without tiers (32 leaves) in place of the first tier.
 static tlfr_status light_trial(const FrameDesc& D, const Ctx& c, int shape, cudaStream_t s, float* ms,
                                std::string& err)
 {

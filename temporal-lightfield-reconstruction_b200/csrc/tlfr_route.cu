@@ -1,8 +1,8 @@
 // tlfr_route.cu — learned routing (no counterpart in the reference: it is the
 // addition that sends easy pixels to a fast path).  The fast path is the plain
 // 1R pass that keeps the first surface when a second one opens instead of
-// refetching at 2R (light_scan_warp in tlfr_query.cu), so the expensive full
-// path runs only where the network is not confident.
+// refetching at 2R (light_unit() in tlfr_query.cu), so the expensive full path
+// runs only where the network is not confident.
 //
 //   features   eight cheap per-pixel features: depth, depth range and CoC
 //              radius in the pixel, depth ranges within 3x3 and 5x5 tiles of
@@ -236,9 +236,10 @@ __device__ __forceinline__ void acc_to_a(const float (&c0)[4], const float (&c1)
 }
 
 // Forward pass of one 16-row tile.  Lane (g = lane/4, t = lane%4) holds rows
-// g and g + 8, whose features are at row[0] and row[1] (zero where not valid).  Outputs: h1, h2 after ReLU, rounded to BF16 (the values the
-// next layer multiplies), columns 8j + 2t (+1); logits y for rows g and g+8
-// (valid on lanes with t == 0).  PAIRS: the features start on 8 bytes, and two are
+// g and g + 8, whose features are at row[0] and row[1] (zero where not valid).
+// Outputs: h1, h2 after ReLU, rounded to BF16 (the values the next layer
+// multiplies), columns 8j + 2t (+1); logits y for rows g and g+8 (valid on lanes
+// with t == 0).  PAIRS: the features start on 8 bytes, and two are
 // loaded at a time (feature_pairs()).
 struct Tile
 {
@@ -294,7 +295,7 @@ __device__ __forceinline__ void tile_forward(const float* __restrict__ P, const 
     {
         float c[4] = { 0, 0, 0, 0 };
 #pragma unroll
-    for (int kk = 0; kk < 4; kk++)
+        for (int kk = 0; kk < 4; kk++)
         {
             uint32_t b0, b1;
             load_b(Wh, kFragW2 + 4 * j + kk, b0, b1);
